@@ -1307,60 +1307,38 @@ extern "C" int32_t qm_expectation_energy(qm_state* st, const qm_pauli_term* term
 
 namespace {
 
-// Targets draw*total on the FP64 chunk prefix, then device searches.  outcomes[i] = index;
-// returns the number of draws near a boundary in *ambiguous.
+// Born-rule draws on the device: one read of the state, the prefix and one search per shot, with a
+// single synchronisation.  outcomes[i] = index; the number of draws near a boundary in *ambiguous.
 int32_t device_sample(qm_state* st, const double* draws, int32_t shots, int64_t* outcomes, int32_t* ambiguous) {
     qm_context* ctx = st->ctx;
-    const uint64_t n = 1ull << st->qubits;
-    uint64_t chunk = std::max<uint64_t>(1024, n / (148 * 8));
-    uint64_t c = 1;
-    while (c < chunk) c <<= 1;
-    if (c > n) c = n;
-    const int blocks = (int)(n / c);
-    size_t need = sizeof(double) * (size_t)blocks           // sums
-                  + sizeof(int64_t) * (size_t)blocks        // last
-                  + sizeof(double) * ((size_t)blocks + 1)   // prefix
-                  + sizeof(double) * (size_t)shots          // targets
-                  + sizeof(int64_t) * 2 * (size_t)shots;    // outcomes + flags
-    int32_t rc = ensure_scratch(ctx, need);
+    const SampleShape g = sample_shape(st->qubits);
+    const size_t fines = (size_t)g.blocks * g.per_block;
+    const size_t result = sizeof(SampleSummary) + sizeof(int64_t) * 2 * (size_t)shots;  // copied back
+    int32_t rc = ensure_scratch(ctx, result + sizeof(double) * (fines + 3 * (size_t)g.blocks + 1 + (size_t)shots));
     if (rc) return rc;
-    rc = ensure_host_scratch(ctx, std::max(sizeof(double) * (size_t)blocks * 2, sizeof(int64_t) * 2 * (size_t)shots) + 64);
+    rc = ensure_host_scratch(ctx, result + sizeof(double) * (size_t)shots);
     if (rc) return rc;
-    char* base = static_cast<char*>(ctx->scratch);
-    double* sums = reinterpret_cast<double*>(base);
-    int64_t* last = reinterpret_cast<int64_t*>(sums + blocks);
-    double* prefix = reinterpret_cast<double*>(last + blocks);
-    double* targets = prefix + blocks + 1;
-    int64_t* out = reinterpret_cast<int64_t*>(targets + shots);
-    int blocks_out = 0, chunk_out = 0;
-    QM_CUDA(launch_block_probs(st->amps, st->qubits, st->precision, sums, last, &blocks_out, &chunk_out, ctx->stream));
-    if (blocks_out != blocks || (uint64_t)chunk_out != c) return fail(QM_E_DEVICE, "sampling chunk mismatch");
-    double* h = ctx->host_scratch;
-    QM_CUDA(cudaMemcpyAsync(h, sums, sizeof(double) * blocks, cudaMemcpyDeviceToHost, ctx->stream));
-    QM_CUDA(cudaMemcpyAsync(h + blocks, last, sizeof(int64_t) * blocks, cudaMemcpyDeviceToHost, ctx->stream));
-    QM_CUDA(cudaStreamSynchronize(ctx->stream));
-    std::vector<double> pre((size_t)blocks + 1);
-    pre[0] = 0;
-    int64_t last_supported = -1;
-    const int64_t* hl = reinterpret_cast<const int64_t*>(h + blocks);
-    for (int b = 0; b < blocks; ++b) {
-        pre[(size_t)b + 1] = pre[(size_t)b] + h[b];
-        last_supported = std::max(last_supported, hl[b]);
-    }
-    double total = pre[(size_t)blocks];
-    if (!std::isfinite(total) || total <= 0) return fail(QM_E_MASS, "The state has no finite positive probability mass.");
-    std::vector<double> tg((size_t)shots);
-    for (int32_t s = 0; s < shots; ++s) tg[(size_t)s] = draws[s] * total;
-    QM_CUDA(cudaMemcpyAsync(prefix, pre.data(), sizeof(double) * (blocks + 1), cudaMemcpyHostToDevice, ctx->stream));
-    QM_CUDA(cudaMemcpyAsync(targets, tg.data(), sizeof(double) * shots, cudaMemcpyHostToDevice, ctx->stream));
-    QM_CUDA(launch_search(st->amps, st->qubits, st->precision, prefix, blocks, (int)c, targets, shots, 1e-12 * total, out,
+    SampleSummary* summary = static_cast<SampleSummary*>(ctx->scratch);
+    int64_t* out = reinterpret_cast<int64_t*>(summary + 1);
+    double* dev_draws = reinterpret_cast<double*>(out + 2 * (size_t)shots);
+    double* fine = dev_draws + shots;
+    double* sums = fine + fines;
+    int64_t* last = reinterpret_cast<int64_t*>(sums + g.blocks);
+    double* prefix = reinterpret_cast<double*>(last + g.blocks);
+    char* host = reinterpret_cast<char*>(ctx->host_scratch);
+    std::memcpy(host + result, draws, sizeof(double) * (size_t)shots);
+    QM_CUDA(cudaMemcpyAsync(dev_draws, host + result, sizeof(double) * (size_t)shots, cudaMemcpyHostToDevice, ctx->stream));
+    QM_CUDA(launch_sample(st->amps, st->precision, g, fine, sums, last, prefix, summary, dev_draws, shots, out,
                           ctx->stream));
-    int64_t* ho = reinterpret_cast<int64_t*>(h);
-    QM_CUDA(cudaMemcpyAsync(ho, out, sizeof(int64_t) * 2 * shots, cudaMemcpyDeviceToHost, ctx->stream));
+    QM_CUDA(cudaMemcpyAsync(host, summary, result, cudaMemcpyDeviceToHost, ctx->stream));
     QM_CUDA(cudaStreamSynchronize(ctx->stream));
+    const SampleSummary* hs = reinterpret_cast<const SampleSummary*>(host);
+    const int64_t* ho = reinterpret_cast<const int64_t*>(hs + 1);
+    if (!std::isfinite(hs->total) || hs->total <= 0)
+        return fail(QM_E_MASS, "The state has no finite positive probability mass.");
     int32_t amb = 0;
     for (int32_t s = 0; s < shots; ++s) {
-        outcomes[s] = ho[s] >= 0 ? ho[s] : last_supported;
+        outcomes[s] = ho[s];
         amb += ho[shots + s] ? 1 : 0;
     }
     if (ambiguous) *ambiguous = amb;

@@ -284,11 +284,20 @@ int expectation_blocks(int qubits);
 cudaError_t launch_pauli_group(const void* amps, int qubits, int precision, uint32_t flip, int terms,
                                const uint32_t* sign, const int32_t* phase, const int32_t* column, int with_mass,
                                int mass_column, int columns, double* partials, cudaStream_t s);
-// Sampling: per-block probability sums, then searches.
-cudaError_t launch_block_probs(const void* amps, int qubits, int precision, double* block_sums,
-                               int64_t* block_last, int* blocks_out, int* chunk_out, cudaStream_t s);
-cudaError_t launch_search(const void* amps, int qubits, int precision, const double* block_prefix,
-                          int blocks, int chunk, const double* targets, int shots, double margin,
+// Sampling: fine and coarse Born masses, their prefix, then one search per shot, all on the stream.
+// out[shot] = outcome, out[shots + shot] = 1 when it lies near a boundary.  `summary` and `out` hold
+// nothing usable when summary->total is not finite and positive.
+struct SampleSummary {
+    double total;
+    int64_t last;  // the last index with mass
+};
+struct SampleShape {
+    uint32_t fine_amps, per_block;  // amplitudes per fine chunk, fine chunks per coarse one
+    int blocks;                     // coarse chunks (at most 2048)
+};
+SampleShape sample_shape(int qubits);
+cudaError_t launch_sample(const void* amps, int precision, const SampleShape& g, double* fine, double* sums,
+                          int64_t* last, double* prefix, SampleSummary* summary, const double* draws, int shots,
                           int64_t* out, cudaStream_t s);
 cudaError_t launch_collapse(void* amps, int qubits, int precision, int64_t outcome, cudaStream_t s);
 // (selected sum, compensation, total sum, compensation) per block for amplitudes with
