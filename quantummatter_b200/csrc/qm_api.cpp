@@ -593,7 +593,7 @@ int32_t device_masses(qm_context* ctx, void* amps, int qubits, int precision, in
     if (rc) return rc;
     double* partial = static_cast<double*>(ctx->scratch);
     int blocks = 0;
-    QM_CUDA(launch_masses(amps, qubits, precision, target, partial, &blocks, ctx->stream));
+    QM_CUDA(launch_split_masses(amps, qubits, precision, 1ull << target, 0, partial, &blocks, ctx->stream));
     double* out = partial + 4 * blocks;
     QM_CUDA(launch_finish_sums(partial, blocks, 4, out, ctx->stream));
     QM_CUDA(cudaMemcpyAsync(ctx->host_scratch, out, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1307,14 +1307,17 @@ extern "C" int32_t qm_expectation_energy(qm_state* st, const qm_pauli_term* term
 
 namespace {
 
-// Born-rule draws on the device: one read of the state, the prefix and one search per shot, with a
-// single synchronisation.  outcomes[i] = index; the number of draws near a boundary in *ambiguous.
-int32_t device_sample(qm_state* st, const double* draws, int32_t shots, int64_t* outcomes, int32_t* ambiguous) {
+// Born-rule draws on the device: one read of the state, the prefix and one search per shot, then
+// `then(summary, partials)` (launches that use the first draw), with a single synchronisation.
+// outcomes[i] = index; the number of draws near a boundary in *ambiguous; the masses in *masses.
+template <typename Then>
+int32_t device_sample(qm_state* st, const double* draws, int32_t shots, int64_t* outcomes, int32_t* ambiguous,
+                      SampleSummary* masses, Then then) {
     qm_context* ctx = st->ctx;
     const SampleShape g = sample_shape(st->qubits);
     const size_t fines = (size_t)g.blocks * g.per_block;
     const size_t result = sizeof(SampleSummary) + sizeof(int64_t) * 2 * (size_t)shots;  // copied back
-    int32_t rc = ensure_scratch(ctx, result + sizeof(double) * (fines + 3 * (size_t)g.blocks + 1 + (size_t)shots));
+    int32_t rc = ensure_scratch(ctx, result + sizeof(double) * (fines + 3 * (size_t)g.blocks + 1 + (size_t)shots + 2 * kReduceBlocksMax));
     if (rc) return rc;
     rc = ensure_host_scratch(ctx, result + sizeof(double) * (size_t)shots);
     if (rc) return rc;
@@ -1330,6 +1333,7 @@ int32_t device_sample(qm_state* st, const double* draws, int32_t shots, int64_t*
     QM_CUDA(cudaMemcpyAsync(dev_draws, host + result, sizeof(double) * (size_t)shots, cudaMemcpyHostToDevice, ctx->stream));
     QM_CUDA(launch_sample(st->amps, st->precision, g, fine, sums, last, prefix, summary, dev_draws, shots, out,
                           ctx->stream));
+    QM_CUDA(then(summary, prefix + g.blocks + 1));
     QM_CUDA(cudaMemcpyAsync(host, summary, result, cudaMemcpyDeviceToHost, ctx->stream));
     QM_CUDA(cudaStreamSynchronize(ctx->stream));
     const SampleSummary* hs = reinterpret_cast<const SampleSummary*>(host);
@@ -1342,8 +1346,11 @@ int32_t device_sample(qm_state* st, const double* draws, int32_t shots, int64_t*
         amb += ho[shots + s] ? 1 : 0;
     }
     if (ambiguous) *ambiguous = amb;
+    if (masses) *masses = *hs;
     return QM_OK;
 }
+
+cudaError_t nothing_more(SampleSummary*, double*) { return cudaSuccess; }
 
 }  // namespace
 
@@ -1355,7 +1362,7 @@ int32_t qm_sample_amplitudes(qm_context* ctx, void* amps, int32_t qubits, int32_
     view.precision = precision;
     view.amps = amps;
     view.bytes = (precision == QM_FP32 ? 8ll : 16ll) << qubits;
-    return device_sample(&view, draws, shots, outcomes, ambiguous);
+    return device_sample(&view, draws, shots, outcomes, ambiguous, nullptr, nothing_more);
 }
 
 extern "C" int32_t qm_sample(qm_state* st, const double* draws, int32_t shots, int64_t* outcomes, int32_t* ambiguous) {
@@ -1367,7 +1374,7 @@ extern "C" int32_t qm_sample(qm_state* st, const double* draws, int32_t shots, i
         if (!std::isfinite(draws[s]) || draws[s] < 0 || draws[s] >= 1) return fail(QM_E_RANGE, "draws must be in [0,1)");
     std::lock_guard<std::recursive_mutex> lock(st->ctx->mu);
     QM_CUDA(cudaSetDevice(st->ctx->device));
-    return device_sample(st, draws, shots, outcomes, ambiguous);
+    return device_sample(st, draws, shots, outcomes, ambiguous, nullptr, nothing_more);
 }
 
 namespace {
@@ -1390,19 +1397,19 @@ int32_t selection_mask(const int32_t* qubits, int32_t count, int32_t register_qu
 // (selected, total) Born masses on the device, FP64 compensated.
 int32_t pattern_masses(qm_state* st, uint64_t mask, uint64_t pattern, double* selected, double* total) {
     qm_context* ctx = st->ctx;
-    int32_t rc = ensure_scratch(ctx, sizeof(double) * (4 * 148 * 4 + 8));
+    int32_t rc = ensure_scratch(ctx, sizeof(double) * (4 * kReduceBlocksMax + 8));
     if (rc) return rc;
     rc = ensure_host_scratch(ctx, 4 * sizeof(double));
     if (rc) return rc;
     double* partial = static_cast<double*>(ctx->scratch);
     int blocks = 0;
-    QM_CUDA(launch_pattern_masses(st->amps, st->qubits, st->precision, mask, pattern, partial, &blocks, ctx->stream));
+    QM_CUDA(launch_split_masses(st->amps, st->qubits, st->precision, mask, pattern, partial, &blocks, ctx->stream));
     double* out = partial + 4 * blocks;
     QM_CUDA(launch_finish_sums(partial, blocks, 4, out, ctx->stream));
     QM_CUDA(cudaMemcpyAsync(ctx->host_scratch, out, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     QM_CUDA(cudaStreamSynchronize(ctx->stream));
     *selected = ctx->host_scratch[0] + ctx->host_scratch[1];
-    *total = ctx->host_scratch[2] + ctx->host_scratch[3];
+    *total = *selected + (ctx->host_scratch[2] + ctx->host_scratch[3]);
     return QM_OK;
 }
 
@@ -1437,16 +1444,17 @@ extern "C" int32_t qm_measure(qm_state* st, const int32_t* qubits, int32_t count
     if (!std::isfinite(u) || u < 0 || u >= 1) return fail(QM_E_RANGE, "draw must be in [0,1)");
     std::lock_guard<std::recursive_mutex> lock(st->ctx->mu);
     QM_CUDA(cudaSetDevice(st->ctx->device));
-    // one full-basis Born draw (the device CDF and search of qm_sample)
+    // one full-basis Born draw (qm_sample's), the branch it selects and the projection onto it, all
+    // queued before the host looks at the outcome
     int64_t basis = -1;
     int32_t amb = 0;
-    if ((rc = device_sample(st, &u, 1, &basis, &amb))) return rc;
-    const uint64_t pattern = (uint64_t)basis & mask;
-    double branch = 0, total = 0;
-    if ((rc = pattern_masses(st, mask, pattern, &branch, &total))) return rc;
+    SampleSummary masses;
+    rc = device_sample(st, &u, 1, &basis, &amb, &masses, [&](SampleSummary* summary, double* partials) {
+        return launch_measure(st->amps, st->qubits, st->precision, mask, summary, partials, st->ctx->stream);
+    });
+    if (rc) return rc;
+    const double branch = masses.branch[0] + masses.branch[1];
     if (!std::isfinite(branch) || branch <= 0) return fail(QM_E_MASS, "The state has no finite positive probability mass.");
-    QM_CUDA(launch_project(st->amps, st->qubits, st->precision, mask, pattern, std::sqrt(branch), st->ctx->stream));
-    QM_CUDA(cudaStreamSynchronize(st->ctx->stream));
     int32_t out = 0;
     for (int32_t k = 0; k < count; ++k) out |= (int32_t)((basis >> qubits[k]) & 1) << k;
     *outcome = out;
@@ -1463,10 +1471,10 @@ extern "C" int32_t qm_measure_all(qm_state* st, double u, int64_t* outcome, int3
     QM_CUDA(cudaSetDevice(st->ctx->device));
     int64_t out = -1;
     int32_t amb = 0;
-    rc = device_sample(st, &u, 1, &out, &amb);
+    rc = device_sample(st, &u, 1, &out, &amb, nullptr, [&](SampleSummary* summary, double*) {
+        return launch_collapse(st->amps, st->qubits, st->precision, summary, st->ctx->stream);
+    });
     if (rc) return rc;
-    QM_CUDA(launch_collapse(st->amps, st->qubits, st->precision, out, st->ctx->stream));
-    QM_CUDA(cudaStreamSynchronize(st->ctx->stream));
     *outcome = out;
     if (ambiguous) *ambiguous = amb;
     return QM_OK;

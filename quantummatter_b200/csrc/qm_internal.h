@@ -262,9 +262,10 @@ cudaError_t launch_plan_pass(const Plan& plan, size_t pass, void* amps, const Fu
 cudaError_t launch_reset(void* amps, int qubits, int precision, cudaStream_t s);
 cudaError_t launch_convert_from_f64(void* dst_f32, const double* src_f64, int64_t n, cudaStream_t s);
 cudaError_t launch_convert_to_f64(double* dst_f64, const void* src_f32, int64_t n, cudaStream_t s);
-// FP64 partial sums: writes `blocks` partial (sum, compensation) pairs into scratch.
-cudaError_t launch_masses(const void* amps, int qubits, int precision, int target, double* scratch,
-                          int* blocks_out, cudaStream_t s);
+// FP64 masses of the amplitudes with (index & mask) == pattern and of the others: (sum, compensation)
+// of each per block into scratch, at most kReduceBlocksMax blocks.
+cudaError_t launch_split_masses(const void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern,
+                                double* scratch, int* blocks_out, cudaStream_t s);
 cudaError_t launch_pauli(void* amps, int qubits, int precision, int target, int pauli, cudaStream_t s);
 cudaError_t launch_damping(void* amps, int qubits, int precision, int target, int jump, double scale,
                            double jump_scale, double stay_scale, cudaStream_t s);
@@ -289,7 +290,9 @@ cudaError_t launch_pauli_group(const void* amps, int qubits, int precision, uint
 // nothing usable when summary->total is not finite and positive.
 struct SampleSummary {
     double total;
-    int64_t last;  // the last index with mass
+    int64_t last;      // the last index with mass
+    int64_t outcome;   // the first shot's outcome
+    double branch[2];  // a measurement's selected mass (launch_measure): sum, compensation
 };
 struct SampleShape {
     uint32_t fine_amps, per_block;  // amplitudes per fine chunk, fine chunks per coarse one
@@ -299,13 +302,12 @@ SampleShape sample_shape(int qubits);
 cudaError_t launch_sample(const void* amps, int precision, const SampleShape& g, double* fine, double* sums,
                           int64_t* last, double* prefix, SampleSummary* summary, const double* draws, int shots,
                           int64_t* out, cudaStream_t s);
-cudaError_t launch_collapse(void* amps, int qubits, int precision, int64_t outcome, cudaStream_t s);
-// (selected sum, compensation, total sum, compensation) per block for amplitudes with
-// (index & mask) == pattern; blocks = expectation_blocks(qubits).
-cudaError_t launch_pattern_masses(const void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern,
-                                  double* scratch, int* blocks_out, cudaStream_t s);
-cudaError_t launch_project(void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern, double norm,
-                           cudaStream_t s);
+// After launch_sample on the same stream: collapses the state to the first shot's outcome, or
+// projects it onto that outcome's value of the masked bits (the branch mass into summary->branch;
+// partials: 2 * kReduceBlocksMax doubles).  Neither writes without a finite positive mass.
+cudaError_t launch_collapse(void* amps, int qubits, int precision, const SampleSummary* summary, cudaStream_t s);
+cudaError_t launch_measure(void* amps, int qubits, int precision, uint64_t mask, SampleSummary* summary,
+                           double* partials, cudaStream_t s);
 
 // ---------------------------------------------------------------- tiled expectation (qm_expect.cu)
 constexpr int kTileMaxTerms = 256;

@@ -169,29 +169,52 @@ int stream_blocks(uint64_t n) {
 
 // ---------------------------------------------------------------- noise
 
-// Masses of target-zero and target-one amplitudes (CpuNoiseChannelBackend.cs:88-106):
-// compensated FP64 per thread, deterministic block tree; one (zero, one) pair of
-// compensated partials per block.
+// Amplitudes in one 16-byte access, and accesses per thread and round of the streaming reductions.
+template <typename T> constexpr int kPer = 16 / (int)sizeof(typename Vec2<T>::type);
+constexpr int kLoads = 4;
+
+// Born masses of the amplitudes whose masked bits equal `pattern` and of the others: the target-zero
+// and target-one masses of a damping (CpuNoiseChannelBackend.cs:88-106; mask = the target, pattern
+// 0) and a marginal's selected mass with the rest of the total (StateVector.MarginalProbability,
+// StateVector.Observations.cs:10-36).  Compensated FP64 per thread, deterministic block tree, one
+// (sum, compensation) pair of each per block.  Bound by HBM; the state is read in index order with
+// four 16-byte loads per thread in flight, whatever the masked bits are.  Three rounds of a monitored
+// 26-qubit complex128 circuit (damping, marginal, measurement): 8.31 to 7.90 ms, with the branch's own
+// mass and projection below.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_masses(const typename Vec2<T>::type* __restrict__ s, uint32_t pairs,
-                                                     int target, double* out) {
+__global__ void __launch_bounds__(kThreads) k_split_masses(const typename Vec2<T>::type* __restrict__ s, uint64_t n,
+                                                           uint64_t mask, uint64_t pattern, double* out) {
     __shared__ KSum red[kThreads / 32];
-    KSum z{0, 0}, o{0, 0};
-    uint32_t bit = 1u << target;
-    for (uint32_t p = blockIdx.x * kThreads + threadIdx.x; p < pairs; p += gridDim.x * kThreads) {
-        uint32_t f = insert_zero(p, target);
-        Cx<T> x = load_amp<T>(s, f), y = load_amp<T>(s, f | bit);
-        double xr = x.re, xi = x.im, yr = y.re, yi = y.im;
-        z.add(xr * xr + xi * xi);
-        o.add(yr * yr + yi * yi);
+    KSum sel{0, 0}, rest{0, 0};
+    const uint64_t loads = n / kPer<T>;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * (kThreads * kLoads) + threadIdx.x; i0 < loads;
+         i0 += (uint64_t)gridDim.x * (kThreads * kLoads)) {
+        __align__(16) T v[kLoads][2 * kPer<T>];
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j)
+            if (i0 + j * kThreads < loads)
+                *reinterpret_cast<uint4*>(v[j]) = __ldg(reinterpret_cast<const uint4*>(s) + i0 + j * kThreads);
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+            if (i0 + j * kThreads >= loads) break;
+#pragma unroll
+            for (int u = 0; u < kPer<T>; ++u) {
+                const double re = v[j][2 * u], im = v[j][2 * u + 1];
+                const bool on = (((i0 + j * kThreads) * kPer<T> + u) & mask) == pattern;
+                KSum a = on ? sel : rest;
+                a.add(re * re + im * im);
+                sel = on ? a : sel;
+                rest = on ? rest : a;
+            }
+        }
     }
-    KSum zt = block_reduce_ksum(z, red);
-    KSum ot = block_reduce_ksum(o, red);
+    const KSum st = block_reduce_ksum(sel, red);
+    const KSum rt = block_reduce_ksum(rest, red);
     if (threadIdx.x == 0) {
-        out[4 * blockIdx.x + 0] = zt.s;
-        out[4 * blockIdx.x + 1] = zt.c;
-        out[4 * blockIdx.x + 2] = ot.s;
-        out[4 * blockIdx.x + 3] = ot.c;
+        out[4 * blockIdx.x + 0] = st.s;
+        out[4 * blockIdx.x + 1] = st.c;
+        out[4 * blockIdx.x + 2] = rt.s;
+        out[4 * blockIdx.x + 3] = rt.c;
     }
 }
 
@@ -313,15 +336,15 @@ __global__ void __launch_bounds__(kThreads) k_pauli_group(const typename Vec2<T>
     }
 }
 
-// Column sums of a [rows][columns] table in fixed order: one warp per column.
-__global__ void k_finish_sums(const double* __restrict__ partials, int rows, int columns, double* out) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (warp >= columns) return;
+// Column sums of a [rows][columns] table in fixed order: one block per column, so that the few
+// hundred rows of a reduction are four or five loads per thread and not a chain of twenty.
+__global__ void __launch_bounds__(128) k_finish_sums(const double* __restrict__ partials, int rows, int columns,
+                                                     double* out) {
+    __shared__ KSum red[4];
     KSum acc{0, 0};
-    for (int r = lane; r < rows; r += 32) acc.add(partials[(size_t)r * columns + warp]);
-    for (int d = 16; d > 0; d >>= 1) acc.merge(shfl_down_ksum(acc, d));
-    if (lane == 0) out[warp] = acc.value();
+    for (int r = threadIdx.x; r < rows; r += 128) acc.add(partials[(size_t)r * columns + blockIdx.x]);
+    acc = block_reduce_ksum(acc, red);
+    if (threadIdx.x == 0) out[blockIdx.x] = acc.value();
 }
 
 // ---------------------------------------------------------------- sampling
@@ -330,8 +353,9 @@ __global__ void k_finish_sums(const double* __restrict__ partials, int rows, int
 // amplitudes, one warp each, and coarse chunks of `per_block` fine ones, one block each.  A shot
 // then reads the coarse prefix, the fine masses of one coarse chunk and the amplitudes of one fine
 // chunk.  The pass is bound by HBM: 1000 shots of a 27-qubit complex128 state take 0.40 ms with all
-// launches, 0.33 of them the state's read at the copy rate.  512 amplitudes a fine chunk keep 16 (complex64: 8) independent 16-byte loads per lane in flight and the table at
-// 1/1024 of a complex128 state's bytes.
+// launches, 0.33 of them the state's read at the copy rate.  512 amplitudes a fine chunk keep 16
+// (complex64: 8) independent 16-byte loads per lane in flight and the table at 1/1024 of a
+// complex128 state's bytes.
 constexpr int kFineAmps = 512;
 
 template <typename T>
@@ -346,21 +370,20 @@ __global__ void __launch_bounds__(kThreads) k_cdf_chunks(const typename Vec2<T>:
         const uint32_t chunk = blockIdx.x * per_block + f;
         KSum acc{0, 0};
         if (fine_amps == kFineAmps) {
-            constexpr int kPer = 16 / sizeof(typename Vec2<T>::type);  // amplitudes per 16-byte load
-            constexpr int kLoads = kFineAmps / (32 * kPer);
-            const uint32_t first = chunk * (kFineAmps / kPer) + lane;
-            __align__(16) T v[kLoads][2 * kPer];
+            constexpr int kFineLoads = kFineAmps / (32 * kPer<T>);
+            const uint32_t first = chunk * (kFineAmps / kPer<T>) + lane;
+            __align__(16) T v[kFineLoads][2 * kPer<T>];
 #pragma unroll
-            for (int j = 0; j < kLoads; ++j)
+            for (int j = 0; j < kFineLoads; ++j)
                 *reinterpret_cast<uint4*>(v[j]) = __ldg(reinterpret_cast<const uint4*>(s) + first + 32 * j);
 #pragma unroll
-            for (int j = 0; j < kLoads; ++j)
+            for (int j = 0; j < kFineLoads; ++j)
 #pragma unroll
-                for (int u = 0; u < kPer; ++u) {
+                for (int u = 0; u < kPer<T>; ++u) {
                     const double re = v[j][2 * u], im = v[j][2 * u + 1];
                     const double p = re * re + im * im;
                     acc.add(p);
-                    if (p > 0) my_last = (int64_t)(first + 32 * j) * kPer + u;
+                    if (p > 0) my_last = (int64_t)(first + 32 * j) * kPer<T> + u;
                 }
         } else {
             for (uint32_t i = lane; i < fine_amps; i += 32) {
@@ -489,8 +512,8 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_cdf_search(const typename Vec2<T>::type* __restrict__ s, uint32_t fine_amps,
                                                     uint32_t per_block, int blocks, const double* __restrict__ fine,
                                                     const double* __restrict__ sums, const double* __restrict__ prefix,
-                                                    const SampleSummary* __restrict__ summary,
-                                                    const double* __restrict__ draws, int shots, int64_t* out) {
+                                                    SampleSummary* summary, const double* __restrict__ draws,
+                                                    int shots, int64_t* out) {
     const int shot = (int)(blockIdx.x * 4u + (threadIdx.x >> 5));
     const uint32_t lane = threadIdx.x & 31;
     if (shot >= shots) return;
@@ -548,53 +571,95 @@ __global__ void __launch_bounds__(128) k_cdf_search(const typename Vec2<T>::type
     if (lane == 0) {
         out[shot] = found >= 0 ? found : summary->last;
         out[shots + shot] = ambiguous || found < 0;
+        if (shot == 0) summary->outcome = out[shot];
     }
 }
 
-// Born masses of the amplitudes whose masked bits equal `pattern` and of all amplitudes
-// (StateVector.MarginalProbability and Measure's branch mass, StateVector.Observations.cs:10-88):
-// compensated FP64 per thread, deterministic block tree, (selected, total) per block.
+// The mass of the branch a measurement selected: only the amplitudes whose masked bits equal the
+// outcome's are visited (the item index gets zeros inserted at the masked bits, ascending), so a
+// measurement of c qubits reads 1/2^c of the state.
+struct BranchLaunch {
+    uint64_t mask;
+    uint32_t items;  // 2^(qubits - masked bits)
+    int32_t npos;
+    int32_t pos[32];
+};
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_pattern_masses(const typename Vec2<T>::type* __restrict__ s, uint64_t n,
-                                                             uint64_t mask, uint64_t pattern, double* out) {
+__global__ void __launch_bounds__(kThreads) k_branch_mass(const typename Vec2<T>::type* __restrict__ s,
+                                                          const BranchLaunch L, const SampleSummary* __restrict__ summary,
+                                                          double* out) {
     __shared__ KSum red[kThreads / 32];
-    KSum sel{0, 0}, tot{0, 0};
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kThreads) {
-        const Cx<T> x = load_amp<T>(s, i);
-        const double xr = x.re, xi = x.im;
-        const double p = xr * xr + xi * xi;
-        tot.add(p);
-        if ((i & mask) == pattern) sel.add(p);
+    KSum acc{0, 0};
+    const uint32_t pattern = (uint32_t)((uint64_t)summary->outcome & L.mask);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * (kThreads * kLoads) + threadIdx.x; i0 < L.items;
+         i0 += (uint64_t)gridDim.x * (kThreads * kLoads)) {
+        uint32_t x[kLoads];
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) x[j] = (uint32_t)i0 + j * kThreads;
+        for (int k = 0; k < L.npos; ++k)
+#pragma unroll
+            for (int j = 0; j < kLoads; ++j) x[j] = insert_zero(x[j], L.pos[k]);
+        Cx<T> v[kLoads];
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j)
+            v[j] = i0 + j * kThreads < L.items ? load_amp<T>(s, x[j] | pattern) : Cx<T>{(T)0, (T)0};
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+            const double re = v[j].re, im = v[j].im;
+            acc.add(re * re + im * im);
+        }
     }
-    KSum st = block_reduce_ksum(sel, red);
-    KSum tt = block_reduce_ksum(tot, red);
+    acc = block_reduce_ksum(acc, red);
     if (threadIdx.x == 0) {
-        out[4 * blockIdx.x + 0] = st.s;
-        out[4 * blockIdx.x + 1] = st.c;
-        out[4 * blockIdx.x + 2] = tt.s;
-        out[4 * blockIdx.x + 3] = tt.c;
+        out[2 * blockIdx.x + 0] = acc.s;
+        out[2 * blockIdx.x + 1] = acc.c;
     }
 }
 
 // Measure's projection (StateVector.Observations.cs:86-93): the matching branch divided by the
-// square root of its mass, every other amplitude zero.
+// square root of its mass, every other amplitude zero.  Only the branch is read; a branch or total
+// without finite positive mass leaves the state as it is.  Bound by HBM: one write of the state and
+// one read of the branch.
 template <typename T>
-__global__ void k_project(typename Vec2<T>::type* s, uint64_t n, uint64_t mask, uint64_t pattern, double norm) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        Cx<T> x = load_amp<T>(s, i);
-        if ((i & mask) == pattern) {
-            x.re = (T)((double)x.re / norm);
-            x.im = (T)((double)x.im / norm);
-        } else {
-            x.re = (T)0;
-            x.im = (T)0;
+__global__ void __launch_bounds__(kThreads) k_project(typename Vec2<T>::type* s, uint64_t n, uint64_t mask,
+                                                      const SampleSummary* __restrict__ summary) {
+    const double mass = summary->branch[0] + summary->branch[1];
+    if (!(summary->total > 0.0 && isfinite(summary->total) && mass > 0.0 && isfinite(mass))) return;
+    const double norm = sqrt(mass);
+    const uint64_t pattern = (uint64_t)summary->outcome & mask;
+    const uint64_t loads = n / kPer<T>;
+    uint4* p = reinterpret_cast<uint4*>(s);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * (kThreads * kLoads) + threadIdx.x; i0 < loads;
+         i0 += (uint64_t)gridDim.x * (kThreads * kLoads)) {
+        __align__(16) T v[kLoads][2 * kPer<T>];
+        bool on[kLoads][kPer<T>];
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+            const uint64_t i = i0 + j * kThreads;
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < kPer<T>; ++u) any |= on[j][u] = ((i * kPer<T> + u) & mask) == pattern;
+            if (i < loads && any) *reinterpret_cast<uint4*>(v[j]) = p[i];
         }
-        store_amp<T>(s, i, x);
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+            const uint64_t i = i0 + j * kThreads;
+#pragma unroll
+            for (int u = 0; u < kPer<T>; ++u) {
+                v[j][2 * u] = on[j][u] ? (T)((double)v[j][2 * u] / norm) : (T)0;
+                v[j][2 * u + 1] = on[j][u] ? (T)((double)v[j][2 * u + 1] / norm) : (T)0;
+            }
+            if (i < loads) p[i] = *reinterpret_cast<const uint4*>(v[j]);
+        }
     }
 }
 
+// MeasureAll's collapse onto the drawn basis state; no write without a drawn outcome.
 template <typename T>
-__global__ void k_collapse(typename Vec2<T>::type* s, uint64_t n, uint64_t outcome) {
+__global__ void k_collapse(typename Vec2<T>::type* s, uint64_t n, const SampleSummary* __restrict__ summary) {
+    if (!(summary->total > 0.0 && isfinite(summary->total))) return;
+    const uint64_t outcome = (uint64_t)summary->outcome;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (; i < n; i += stride) store_amp<T>(s, i, Cx<T>{i == outcome ? (T)1 : (T)0, (T)0});
@@ -630,13 +695,15 @@ static int reduce_blocks(uint64_t items) {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>(b, (uint64_t)kReduceBlocksMax));
 }
 
-cudaError_t launch_masses(const void* amps, int qubits, int precision, int target, double* scratch, int* blocks_out,
-                          cudaStream_t st) {
-    uint32_t pairs = (uint32_t)((1ull << qubits) >> 1);
-    int blocks = reduce_blocks(pairs);
+cudaError_t launch_split_masses(const void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern,
+                                double* scratch, int* blocks_out, cudaStream_t st) {
+    const uint64_t n = 1ull << qubits;
+    const int blocks = reduce_blocks(n);
     *blocks_out = blocks;
-    if (precision == QM_FP32) k_masses<float><<<blocks, kThreads, 0, st>>>((const float2*)amps, pairs, target, scratch);
-    else k_masses<double><<<blocks, kThreads, 0, st>>>((const double2*)amps, pairs, target, scratch);
+    if (precision == QM_FP32)
+        k_split_masses<float><<<blocks, kThreads, 0, st>>>((const float2*)amps, n, mask, pattern, scratch);
+    else
+        k_split_masses<double><<<blocks, kThreads, 0, st>>>((const double2*)amps, n, mask, pattern, scratch);
     return cudaGetLastError();
 }
 
@@ -741,9 +808,7 @@ cudaError_t launch_pauli_group(const void* amps, int qubits, int precision, uint
 }
 
 cudaError_t launch_finish_sums(const double* partials, int rows, int columns, double* out, cudaStream_t st) {
-    int threads = 128;
-    int blocks = (columns * 32 + threads - 1) / threads;
-    k_finish_sums<<<blocks, threads, 0, st>>>(partials, rows, columns, out);
+    k_finish_sums<<<columns, 128, 0, st>>>(partials, rows, columns, out);
     return cudaGetLastError();
 }
 
@@ -778,32 +843,32 @@ cudaError_t launch_sample(const void* amps, int precision, const SampleShape& g,
     return cudaGetLastError();
 }
 
-cudaError_t launch_pattern_masses(const void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern,
-                                  double* scratch, int* blocks_out, cudaStream_t st) {
+cudaError_t launch_measure(void* amps, int qubits, int precision, uint64_t mask, SampleSummary* summary,
+                           double* partials, cudaStream_t st) {
     const uint64_t n = 1ull << qubits;
-    const int blocks = reduce_blocks(n);
-    *blocks_out = blocks;
-    if (precision == QM_FP32)
-        k_pattern_masses<float><<<blocks, kThreads, 0, st>>>((const float2*)amps, n, mask, pattern, scratch);
-    else
-        k_pattern_masses<double><<<blocks, kThreads, 0, st>>>((const double2*)amps, n, mask, pattern, scratch);
+    BranchLaunch L{};
+    L.mask = mask;
+    for (int b = 0; b < qubits; ++b)
+        if ((mask >> b) & 1) L.pos[L.npos++] = b;
+    L.items = (uint32_t)(n >> L.npos);
+    const int blocks = reduce_blocks(L.items);
+    const unsigned grid = (unsigned)std::max(1, stream_blocks((n + kLoads - 1) / kLoads));
+    if (precision == QM_FP32) {
+        k_branch_mass<float><<<blocks, kThreads, 0, st>>>((const float2*)amps, L, summary, partials);
+        k_finish_sums<<<2, 128, 0, st>>>(partials, blocks, 2, summary->branch);
+        k_project<float><<<grid, kThreads, 0, st>>>((float2*)amps, n, mask, summary);
+    } else {
+        k_branch_mass<double><<<blocks, kThreads, 0, st>>>((const double2*)amps, L, summary, partials);
+        k_finish_sums<<<2, 128, 0, st>>>(partials, blocks, 2, summary->branch);
+        k_project<double><<<grid, kThreads, 0, st>>>((double2*)amps, n, mask, summary);
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_project(void* amps, int qubits, int precision, uint64_t mask, uint64_t pattern, double norm,
-                           cudaStream_t st) {
-    const uint64_t n = 1ull << qubits;
-    if (precision == QM_FP32)
-        k_project<float><<<stream_blocks(n), kThreads, 0, st>>>((float2*)amps, n, mask, pattern, norm);
-    else
-        k_project<double><<<stream_blocks(n), kThreads, 0, st>>>((double2*)amps, n, mask, pattern, norm);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_collapse(void* amps, int qubits, int precision, int64_t outcome, cudaStream_t st) {
+cudaError_t launch_collapse(void* amps, int qubits, int precision, const SampleSummary* summary, cudaStream_t st) {
     uint64_t n = 1ull << qubits;
-    if (precision == QM_FP32) k_collapse<float><<<stream_blocks(n), kThreads, 0, st>>>((float2*)amps, n, (uint64_t)outcome);
-    else k_collapse<double><<<stream_blocks(n), kThreads, 0, st>>>((double2*)amps, n, (uint64_t)outcome);
+    if (precision == QM_FP32) k_collapse<float><<<stream_blocks(n), kThreads, 0, st>>>((float2*)amps, n, summary);
+    else k_collapse<double><<<stream_blocks(n), kThreads, 0, st>>>((double2*)amps, n, summary);
     return cudaGetLastError();
 }
 

@@ -8,6 +8,7 @@ import pytest
 import oracle as orc
 from circuits import random_state
 from quantummatter_b200.backend import FP32, FP64, DeviceState
+from quantummatter_b200.errors import MassError
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +54,38 @@ def test_draws_of_a_basis_state(gpu_context):
             st.Upload(psi)
             got, _ = st.Sample([0.0, 0.25, 1 - 2.0 ** -53])
         assert list(got) == [k, k, k]
+
+
+@pytest.mark.parametrize("precision,tol", [(FP64, 1e-12), (FP32, 2e-6)], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("n", [1, 2, 5, 11, 13])
+def test_projection_onto_any_selection(gpu_context, n, precision, tol):
+    """The branch's amplitudes are enumerated by their free bits: single qubits from lowest to highest,
+    neighbours, scattered selections and the whole register."""
+    psi = random_state(n, 40 + n) * 1.7
+    rng = np.random.default_rng(n)
+    selections = [[0], [n - 1], list(range(n)), sorted(rng.choice(n, size=(n + 1) // 2, replace=False).tolist())]
+    for qubits in selections:
+        u = float(rng.random())
+        with DeviceState(gpu_context, n, precision) as st:
+            st.Upload(psi)
+            m0, m1 = st.QubitMasses(qubits[-1])
+            outcome, _ = st.Measure(qubits, u)
+            got = st.Download()
+        bit = (np.arange(1 << n) >> qubits[-1]) & 1
+        p = np.abs(psi) ** 2
+        assert abs(m0 - p[bit == 0].sum()) <= tol * p.sum() and abs(m1 - p[bit == 1].sum()) <= tol * p.sum()
+        want_state, want = orc.measure(psi, qubits, u)
+        assert outcome == want
+        assert np.max(np.abs(got - want_state)) <= tol
+
+
+def test_a_state_without_mass_is_left_alone(gpu_context):
+    for bad in (0.0, np.inf, np.nan):
+        psi = np.full(1 << 10, bad, dtype=np.complex128)
+        with DeviceState(gpu_context, 10, FP64) as st:
+            st.Upload(psi)
+            for call in (lambda: st.Sample([0.5]), lambda: st.Measure([3], 0.5), lambda: st.MeasureAll(0.5),
+                         lambda: st.MarginalProbability([2], 1)):
+                with pytest.raises(MassError):
+                    call()
+            assert np.array_equal(st.Download(), psi, equal_nan=True)
