@@ -333,7 +333,7 @@ int32_t run_plan(qm_context* ctx, const Plan& plan, void* amps, const volatile i
                 QM_CUDA(launch_dense_tc(amps, plan.qubits, op, plan.d_dense_tc + op.tc_image, plan.d_status,
                                         ctx->sm_count, ctx->stream));
             else
-                QM_CUDA(launch_dense(amps, plan.qubits, plan.precision, op,
+                QM_CUDA(launch_dense(amps, plan.qubits, plan.precision, op, plan.dense_matrices.data() + 2 * op.matrix,
                                      reinterpret_cast<const double2*>(plan.d_dense) + op.matrix, plan.d_status,
                                      ctx->sm_count, ctx->stream));
             int32_t rc = chunk_boundary();

@@ -2,8 +2,13 @@
 //
 // A fused gate on m <= 6 qubits Q is a dense 2^m x 2^m unitary U applied to every column of the
 // state: out(a, c) = sum_b U(a, b) in(b, c), where b, a enumerate the Q bits and c the others.
-// A CTA tile holds 2^m rows and 2^c columns (m + c = 12, 4096 amplitudes): the columns are the
-// lowest c index bits outside Q, so global memory is read in runs.
+// Gates of up to four qubits run on k_dense_reg and complex128 ones of five and six on k_dense_mma
+// (qm_dense_direct.cu); complex64 gates of five and six run on the tensor cores (qm_dense_tc.cu).
+// This file holds the choice, the tensor maps and what is left for k_dense: complex64 gates of five
+// and six qubits on the FP32 pipes (states under 11 qubits, or QM_DENSE_TC=0).
+//
+// A CTA tile of k_dense holds 2^m rows and 2^c columns (m + c = 12, 4096 amplitudes): the columns are
+// the lowest c index bits outside Q, so global memory is read in runs.
 //
 // Staging: the tile travels between HBM and shared memory by bulk copies (cp.async.bulk, the TMA
 // unit's untiled form) that complete on an mbarrier, in a ring of 2-4 buffers: while the CTA
@@ -12,10 +17,9 @@
 // run every column bit lies below every Q bit; runs of 128 bytes or more are spaced 16 bytes apart
 // in shared memory, so the column accesses of a warp hit distinct banks.
 //
-// Arithmetic: each of the 256 threads owns a 4 x 4 block of (row, column) outputs (2 x 8 for
-// m = 1) and walks b over the 2^m rows of the tile: four complex FMAs per output and step, with
-// U(a, b) for consecutive a read as one row of the transposed unitary (a broadcast within the
-// warp's rows).  Complex128 states compute in FP64, complex64 states in FP32.
+// Arithmetic: each of the 256 threads owns a 4 x 4 block of (row, column) outputs and walks b over
+// the 2^m rows of the tile: four complex FMAs per output and step, with U(a, b) for consecutive a
+// read as one row of the transposed unitary (a broadcast within the warp's rows).
 //
 // Every wait on an mbarrier is bounded (about a second of clock cycles); a wait that runs out
 // records QM_E_TIMEOUT in the launch's status word and the CTA waits, again bounded, for its own
@@ -172,9 +176,9 @@ __global__ void __launch_bounds__(kDenseThreads, 1)
     k_dense(typename Vec2<T>::type* __restrict__ s, const __grid_constant__ DenseLaunch P) {
     using V = typename Vec2<T>::type;
     constexpr int D = 1 << M;
-    constexpr int RA = D < 4 ? D : 4;  // rows per thread
-    constexpr int RC = 16 / RA;        // columns per thread
-    constexpr int RG = D / RA;         // row groups
+    constexpr int RA = 4;       // rows per thread
+    constexpr int RC = 4;       // columns per thread
+    constexpr int RG = D / RA;  // row groups
     extern __shared__ __align__(128) unsigned char smem[];
     V* U = reinterpret_cast<V*>(smem);                                   // [b][a]
     int* wq = reinterpret_cast<int*>(smem + sizeof(V) * D * D);          // [b]
@@ -350,20 +354,6 @@ cudaError_t launch_dense_m(void* amps, const DenseLaunch& P, int grid, int threa
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_dense_t(void* amps, int m, const DenseLaunch& P, int grid, int threads, size_t smem,
-                           cudaStream_t st) {
-    switch (m) {
-    case 1: return launch_dense_m<T, 1>(amps, P, grid, threads, smem, st);
-    case 2: return launch_dense_m<T, 2>(amps, P, grid, threads, smem, st);
-    case 3: return launch_dense_m<T, 3>(amps, P, grid, threads, smem, st);
-    case 4: return launch_dense_m<T, 4>(amps, P, grid, threads, smem, st);
-    case 5: return launch_dense_m<T, 5>(amps, P, grid, threads, smem, st);
-    case 6: return launch_dense_m<T, 6>(amps, P, grid, threads, smem, st);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -507,12 +497,14 @@ bool dense_geometry(int qubits, int precision, const DenseOp& op, DenseGeometry&
 
 std::atomic<int64_t> g_dense_launches{0}, g_dense_tc_launches{0};
 
-cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& op, const double2* matrix,
-                         int32_t* status, int sm_count, cudaStream_t st) {
+cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& op, const double* host_matrix,
+                         const double2* matrix, int32_t* status, int sm_count, cudaStream_t st) {
+    g_dense_launches.fetch_add(1, std::memory_order_relaxed);
+    if (op.m <= 4) return launch_dense_reg(amps, qubits, precision, op, host_matrix, st);
+    if (precision == QM_FP64 && qubits >= 9) return launch_dense_mma(amps, qubits, op, matrix, sm_count, st);
     uint32_t qmask = 0;
     for (int i = 0; i < op.m; ++i) qmask |= 1u << op.q[i];
     if (qubits < 9) {
-        g_dense_launches.fetch_add(1, std::memory_order_relaxed);
         if (precision == QM_FP32)
             k_dense_small<float><<<1, 256, 0, st>>>(reinterpret_cast<float2*>(amps), matrix, qmask, op.m, qubits);
         else
@@ -566,11 +558,10 @@ cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& o
     P.buf_elems = g.buf_elems;
     P.buf_offset = g.buf_offset;
     const int grid = (int)std::min<uint64_t>(g.items, (uint64_t)std::max(1, sm_count));
-    g_dense_launches.fetch_add(1, std::memory_order_relaxed);
     // 16 outputs per thread: 256 threads for a 4096-amplitude tile, 32 for the 512 of a 9-qubit state
     const int threads = 1 << (g.cols_bits + op.m - 4);
-    if (precision == QM_FP32) return launch_dense_t<float>(amps, op.m, P, grid, threads, g.smem, st);
-    return launch_dense_t<double>(amps, op.m, P, grid, threads, g.smem, st);
+    return op.m == 5 ? launch_dense_m<float, 5>(amps, P, grid, threads, g.smem, st)
+                     : launch_dense_m<float, 6>(amps, P, grid, threads, g.smem, st);
 }
 
 }  // namespace qm

@@ -59,6 +59,12 @@ __device__ __forceinline__ uint32_t deposit(uint32_t value, uint32_t mask) {
     return out;
 }
 
+// deposit(v + w, mask) from deposit(v, mask) and deposit(w, mask): the bits outside the mask are set,
+// so that carries cross them.
+__device__ __forceinline__ uint32_t deposit_add(uint32_t v, uint32_t w, uint32_t mask) {
+    return ((v | ~mask) + w) & mask;
+}
+
 // One tensor-map box (cp.async.bulk.tensor) between global and shared memory: `map` is the address
 // of a __grid_constant__ CUtensorMap, `rank` its dimensions (1..5), c the box coordinates.  The load
 // completes on the mbarrier at shared address `bar`; the store joins the thread's bulk group.

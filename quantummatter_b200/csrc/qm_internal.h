@@ -190,7 +190,7 @@ bool plan_dense(const std::vector<qm_gate>& gates, int qubits, int precision, in
                 std::string& error);
 bool dense_geometry(int qubits, int precision, const DenseOp& op, DenseGeometry& g);
 // Tiles of dense fused gates move as tensor-map boxes (cp.async.bulk.tensor) where their bit runs
-// form at most five dimensions; QM_DENSE_TMA=0 keeps them on plain bulk copies.
+// form at most five dimensions; QM_DENSE_TMA=0 keeps them on plain copies.
 constexpr int kDenseTmaMaxRank = 5;
 bool dense_tma_enabled();
 // Tensor-map dimensions of a tile (the runs of tile and outer index bits from bit 0 up); false when
@@ -200,8 +200,14 @@ bool tile_map_dims(uint32_t tile_mask, int qubits, int32_t* lo, int32_t* len, in
 bool encode_tile_map(CUtensorMap* map, void* amps, int precision, int rank, const int32_t* lo, const int32_t* len,
                      const int32_t* tile);
 // One dense fused gate on a state (qm_dense.cu); `matrix` is its transposed unitary in device memory.
-cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& op, const double2* matrix,
-                         int32_t* status, int sm_count, cudaStream_t s);
+cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& op, const double* host_matrix,
+                         const double2* matrix, int32_t* status, int sm_count, cudaStream_t st);
+// Gates of up to four qubits, any state (the unitary travels as a kernel parameter) / complex128
+// gates of five and six qubits in states of at least nine (qm_dense_direct.cu).
+cudaError_t launch_dense_reg(void* amps, int qubits, int precision, const DenseOp& op, const double* matrix,
+                             cudaStream_t st);
+cudaError_t launch_dense_mma(void* amps, int qubits, const DenseOp& op, const double2* matrix, int sm_count,
+                             cudaStream_t st);
 // 6-qubit fused gates on complex64 states of at least 11 qubits run on the tensor cores
 // (qm_dense_tc.cu, 3xTF32) when QM_DENSE_TC=1; otherwise they stay on the FP32 pipes.
 bool dense_tc_enabled();
