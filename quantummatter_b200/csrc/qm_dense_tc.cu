@@ -14,9 +14,11 @@
 // three products hi*hi + hi*lo + lo*hi (the 3xTF32 scheme).  A's split is done once on the host.
 //
 // Per CTA (one per SM), for a ring of tiles of 64 rows x 32 columns (2048 amplitudes, 16 KiB):
-//   - one tensor-map box (cp.async.bulk.tensor, natural index order) or bulk copies of runs
-//     (cp.async.bulk) stage each tile into one of four buffers, three tiles ahead of the one being
-//     converted, with mbarrier completion;
+//   - each tile is staged in natural index order into one of five buffers, four tiles ahead of the
+//     one being converted, with mbarrier completion: as one tensor-map box (cp.async.bulk.tensor)
+//     where its index bits form at most five runs, else by 16-byte cp.async of four producer warps,
+//     which also write it back (27 qubits, gate on 0, 4, 9, 13, 18 and 24: 33 ms with a bulk copy per
+//     run of two amplitudes, 0.54 ms so; 0.49 ms as boxes on neighbouring qubits);
 //   - all 256 threads split the tile into B_hi / B_lo in the canonical K-major layout of the
 //     MMA (two B buffers, so tile i converts while tile i-1's MMAs run);
 //   - one thread issues the 24 MMAs of the tile (8 K-steps x 3 products, M = 128, N = 64, K = 8)
@@ -43,15 +45,18 @@ namespace {
 constexpr int kTcConsumers = 512;                 // 16 warps: conversion and epilogue
 constexpr int kTcProducerWarp = kTcConsumers / 32;  // tile loads and stores
 constexpr int kTcMmaWarp = kTcProducerWarp + 1;     // TMEM allocation, A into TMEM order, MMAs
-constexpr int kTcThreads = kTcConsumers + 64;
+constexpr int kTcThreads = kTcConsumers + 64;       // tiles as tensor-map boxes
+constexpr int kTcCopyWarps = 4;                     // producer warps without boxes: three after the MMA warp
+constexpr int kTcCopyThreads = kTcThreads + 32 * (kTcCopyWarps - 1);
+constexpr int kTcCopies = 32 / kTcCopyWarps;        // 16-byte copies per producer lane and tile
 constexpr int kTcTileBits = 11;      // 64 rows x 32 columns
 constexpr int kTcCols = 32;          // complex columns per tile
 constexpr int kTcN = 2 * kTcCols;    // real columns of B and D
-constexpr int kTcMaxStages = 5;      // staging buffers (4 where five do not fit)
+constexpr int kTcStages = 5;         // staging buffers
+constexpr int kTcStageElems = 1 << kTcTileBits;
 constexpr int kTmemCols = 4 * kTcN;  // two accumulators, then A_hi and A_lo (64 columns each)
 constexpr int kTmemA = 2 * kTcN;     // first column of A_hi
 constexpr long long kTcWaitCycles = 2000000000ll;
-constexpr size_t kTcSmemMax = 226 * 1024;
 
 // shared-memory layout (bytes)
 constexpr int kAHalf = 128 * 64 * 4;           // one 128 x 64 TF32 operand image: 32 KiB
@@ -63,18 +68,20 @@ constexpr int kBSbo = 16 * kBLbo + 16;         // 2320: column groups skewed by 
 constexpr int kBHalf = (kTcN / 8) * kBSbo;     // one 64 x 64 B image: 18560 B
 constexpr int kOffA = 0;                       // A_hi, A_lo
 constexpr int kOffB = 2 * kAHalf;              // [2 buffers][hi, lo]
-constexpr int kOffStage = kOffB + 4 * kBHalf;  // staging ring, stage_bytes each
+constexpr int kOffStage = kOffB + 4 * kBHalf;  // staging ring
+constexpr size_t kTcSmem = kOffStage + (size_t)kTcStages * kTcStageElems * sizeof(float2);
+static_assert(kTcSmem <= 226 * 1024, "dynamic shared memory of one block per SM");
 
 struct TcLaunch {
-    CUtensorMap tmap;        // the tile as one box (tma_rank > 0), else bulk copies of runs
+    CUtensorMap tmap;        // the tile as one box (tma_rank > 0), else 16-byte copies
     int32_t tma_rank, tma_lo[5], tma_len[5], tma_tile[5];
     const float* a_image;    // A_hi then A_lo, already in the MMA's K-major layout (64 KiB)
     int32_t* status;
     uint64_t items;
-    uint32_t outer_mask, copy_mask;
+    uint32_t outer_mask, tile_mask;
     int32_t q_bits[6];
-    int32_t l_bits[kTcTileBits];
-    int32_t cols_bits, run_bits, copies, stride, stage_elems, stages;
+    int32_t l_bits[kTcTileBits - 6];
+    uint32_t off[32];        // index bits of local index 64 i
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -108,11 +115,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
-}
-__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
-                 "r"(bytes)
-                 : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all bulk groups but the newest have finished reading their shared-memory sources
@@ -177,11 +179,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// staged-tile offset of global index bit g, and offsets (amplitudes) of row b (fused-qubit index) and
+// column j
 __device__ __forceinline__ int tile_weight(const TcLaunch& P, int g) {
-    if (g < P.run_bits) return 1 << g;
-    return P.stride << __popc(P.copy_mask & ((1u << g) - 1u));
+    return 1 << __popc(P.tile_mask & ((1u << g) - 1u));
 }
-// staged-tile offsets (amplitudes) of row b (fused-qubit index) and column j
 __device__ __forceinline__ int row_offset(const TcLaunch& P, int b) {
     int w = 0;
     for (int i = 0; i < 6; ++i)
@@ -190,9 +192,16 @@ __device__ __forceinline__ int row_offset(const TcLaunch& P, int b) {
 }
 __device__ __forceinline__ int col_offset(const TcLaunch& P, int j) {
     int w = 0;
-    for (int k = 0; k < P.cols_bits; ++k)
+    for (int k = 0; k < kTcTileBits - 6; ++k)
         if ((j >> k) & 1) w += tile_weight(P, P.l_bits[k]);
     return w;
+}
+// Where local index j of a tile is staged: boxes are in natural order; copied tiles XOR the low three
+// bits of the 16-byte chunk number with the higher ones, so that rows and columns on any bits spread
+// over the banks (linear over XOR).
+__host__ __device__ __forceinline__ uint32_t copy_chunk(uint32_t c) { return c ^ (((c >> 3) ^ (c >> 6) ^ (c >> 9)) & 7u); }
+__device__ __forceinline__ int staged_at(const TcLaunch& P, int j) {
+    return P.tma_rank ? j : (int)((copy_chunk((uint32_t)j >> 1) << 1) | ((uint32_t)j & 1u));
 }
 // byte offset of (row b, complex column j) in a B image: real part in column n = 2j, imaginary
 // part 16 bytes on (column n + 1 of the same core matrix)
@@ -201,8 +210,11 @@ __device__ __forceinline__ int b_image_offset(int b, int j) {
     return (n & 7) * 16 + (n >> 3) * kBSbo + (b & 3) * 4 + (b >> 2) * kBLbo;
 }
 
+// `at`: where this lane's copies of the tile start (index bits), without boxes.  Local index 2 lane +
+// 64 i: the tile holds index bit 0, so 16 bytes are two amplitudes of it, and its lowest five bits or
+// more, so a warp's copies come in runs of 256 bytes or more.
 __device__ __forceinline__ void issue_load(const TcLaunch& P, const float2* s, float2* buf, uint64_t* bar,
-                                           uint64_t item, int lane) {
+                                           uint64_t item, uint32_t at, int lane, int part) {
     if (P.tma_rank) {
         if (lane == 0) {
             int32_t c[5];
@@ -212,15 +224,18 @@ __device__ __forceinline__ void issue_load(const TcLaunch& P, const float2* s, f
         }
         return;
     }
-    const uint32_t base = deposit((uint32_t)item, P.outer_mask);
-    const uint32_t run_bytes = 8u << P.run_bits;
-    if (lane == 0) mbar_arrive_expect_tx(bar, run_bytes * (uint32_t)P.copies);
-    __syncwarp();
-    for (int x = lane; x < P.copies; x += 32)
-        bulk_load(buf + (size_t)x * P.stride, s + (base | deposit((uint32_t)x, P.copy_mask)), run_bytes, bar);
+    const uint32_t dst = smem_u32(buf);
+#pragma unroll
+    for (int k = 0; k < kTcCopies; ++k) {
+        const int i = part * kTcCopies + k;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * copy_chunk(lane + 32 * i)),
+                     "l"(s + (at | P.off[i])) : "memory");
+    }
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ void issue_store(const TcLaunch& P, float2* s, const float2* buf, uint64_t item, int lane) {
+__device__ __forceinline__ void issue_store(const TcLaunch& P, float2* s, const float2* buf, uint64_t item, uint32_t at,
+                                            int lane, int part) {
     if (P.tma_rank) {
         if (lane == 0) {
             int32_t c[5];
@@ -230,11 +245,14 @@ __device__ __forceinline__ void issue_store(const TcLaunch& P, float2* s, const 
         }
         return;
     }
-    const uint32_t base = deposit((uint32_t)item, P.outer_mask);
-    const uint32_t run_bytes = 8u << P.run_bits;
-    for (int x = lane; x < P.copies; x += 32)
-        bulk_store(s + (base | deposit((uint32_t)x, P.copy_mask)), buf + (size_t)x * P.stride, run_bytes);
-    bulk_commit();
+    // each lane writes back what it copies in, so its next copy into this buffer follows its reads
+    const float4* src = reinterpret_cast<const float4*>(buf);
+    float4 v[kTcCopies];
+#pragma unroll
+    for (int k = 0; k < kTcCopies; ++k) v[k] = src[copy_chunk(lane + 32 * (part * kTcCopies + k))];
+#pragma unroll
+    for (int k = 0; k < kTcCopies; ++k)
+        *reinterpret_cast<float4*>(s + (at | P.off[part * kTcCopies + k])) = v[k];
 }
 
 __device__ __forceinline__ float tf32_head(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
@@ -254,16 +272,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 //   16 consumer warps: convert tile i into B buffer i % 2 once mma[bb] shows tile i - 2's MMAs
 //     done, then the epilogue of tile i - 1 over its own staging buffer.
 template <bool kConvJ>
-__global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__ s, const __grid_constant__ TcLaunch P) {
+__global__ void __launch_bounds__(kTcCopyThreads, 1) k_dense_tc(float2* __restrict__ s, const __grid_constant__ TcLaunch P) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t full[kTcMaxStages], done[kTcMaxStages];
+    __shared__ uint64_t full[kTcStages], done[kTcStages];
     __shared__ uint64_t conv[2], accf[2], mma[2];
     __shared__ uint64_t bar_a;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t S = (uint32_t)P.stages;
+    constexpr uint32_t S = kTcStages;
     float* a_img = reinterpret_cast<float*>(smem + kOffA);
     unsigned char* b_img = smem + kOffB;
     float2* stage = reinterpret_cast<float2*>(smem + kOffStage);
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
     if (t == 0) {
         if (P.tma_rank) tma_prefetch(&P.tmap);
         for (uint32_t k = 0; k < S; ++k) {
-            mbar_init(&full[k], 1);
+            mbar_init(&full[k], P.tma_rank ? 1 : 32 * kTcCopyWarps);  // the box's transaction, or every producer lane
             mbar_init(&done[k], kTcConsumers);
         }
         for (int k = 0; k < 2; ++k) {
@@ -298,25 +316,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
     uint32_t tiles = 0;
     if ((uint64_t)blockIdx.x < P.items) tiles = (uint32_t)((P.items - 1 - blockIdx.x) / step + 1);
 
-    if (warp == kTcProducerWarp) {
-        if (lane == 0) {
+    if (warp == kTcProducerWarp || warp > kTcMmaWarp) {
+        const int part = warp == kTcProducerWarp ? 0 : warp - kTcMmaWarp;
+        if (part == 0 && lane == 0) {
             mbar_arrive_expect_tx(&bar_a, 2u * kAHalf);
             bulk_load(a_img, P.a_image, 2u * kAHalf, &bar_a);
         }
+        // tile starts of the next load and store, advanced by masked additions
+        const uint32_t lane_at = deposit(2u * lane, P.tile_mask), step_at = deposit((uint32_t)step, P.outer_mask);
+        uint32_t store_at = deposit(blockIdx.x, P.outer_mask), load_at = store_at;
         uint32_t issued = 0;
-        for (; issued + 1 < S && issued < tiles; ++issued)
-            issue_load(P, s, stage + (size_t)issued * P.stage_elems, &full[issued], blockIdx.x + issued * step, lane);
+        for (; issued + 1 < S && issued < tiles; ++issued) {
+            issue_load(P, s, stage + (size_t)issued * kTcStageElems, &full[issued], blockIdx.x + issued * step,
+                       load_at | lane_at, lane, part);
+            load_at = deposit_add(load_at, step_at, P.outer_mask);
+        }
         uint32_t b = 0, lap = 0;
         for (uint32_t j = 0; j < tiles; ++j) {
             // lane 0 waits and decides for the warp: 0 go on, 1 another role stopped, 2 timed out
             int st = 0;
             if (lane == 0) st = abort_flag ? 1 : (mbar_wait_bounded(&done[b], lap & 1u) ? 0 : 2);
             st = __shfl_sync(0xffffffffu, st, 0);
+            __syncwarp();  // what lane 0's wait made visible is so for the lanes that copy it out
             if (st) {
                 if (st == 2 && lane == 0) abort_flag = 1;
                 break;
             }
-            issue_store(P, s, stage + (size_t)b * P.stage_elems, blockIdx.x + (uint64_t)j * step, lane);
+            issue_store(P, s, stage + (size_t)b * kTcStageElems, blockIdx.x + (uint64_t)j * step,
+                        store_at | lane_at, lane, part);
+            store_at = deposit_add(store_at, step_at, P.outer_mask);
             const uint32_t n = j + S - 1;
             if (n < tiles) {
                 // the buffer of tile j - 1: all stores but the newest have read their buffers
@@ -324,7 +352,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
                 bulk_wait_read_older();
                 fence_proxy_async();
                 __syncwarp();
-                issue_load(P, s, stage + (size_t)nb * P.stage_elems, &full[nb], blockIdx.x + (uint64_t)n * step, lane);
+                issue_load(P, s, stage + (size_t)nb * kTcStageElems, &full[nb], blockIdx.x + (uint64_t)n * step,
+                           load_at | lane_at, lane, part);
+                load_at = deposit_add(load_at, step_at, P.outer_mask);
                 ++issued;
             }
             if (++b == S) {
@@ -335,6 +365,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
         // no load may still be writing shared memory when the block exits
         for (uint32_t k = issued > S ? issued - S : 0; k < issued; ++k)
             mbar_wait_bounded(&full[k % S], (k / S) & 1u);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         bulk_wait_all();
     } else if (warp == kTcMmaWarp) {
         if (lane == 0) {
@@ -379,7 +410,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
         {
             const int rb = row_offset(P, cb);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) conv_src[k] = rb + col_offset(P, cj + 8 * k);
+            for (int k = 0; k < 4; ++k) conv_src[k] = staged_at(P, rb + col_offset(P, cj + 8 * k));
         }
         const int conv_dst = b_image_offset(cb, cj);
 
@@ -393,7 +424,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
         {
             const int base = row_offset(P, ea) + col_offset(P, 8 * (warp >> 2) + 4 * ep);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) out_off[q] = base + col_offset(P, kConvJ ? ((q + ea) & 3) : q);
+            for (int q = 0; q < 4; ++q) out_off[q] = staged_at(P, base + col_offset(P, kConvJ ? ((q + ea) & 3) : q));
         }
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
@@ -429,7 +460,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
                     abort_flag = 1;
                     break;
                 }
-                const float2* tile = stage + (size_t)cur * P.stage_elems;
+                const float2* tile = stage + (size_t)cur * kTcStageElems;
                 unsigned char* bhi = b_img + (size_t)bb * 2 * kBHalf + conv_dst;
                 unsigned char* blo = bhi + kBHalf;
 #pragma unroll
@@ -501,7 +532,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(float2* __restrict__
                         o[3] = x1;
                     }
                 }
-                float2* out = stage + (size_t)prev * P.stage_elems;
+                float2* out = stage + (size_t)prev * kTcStageElems;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) out[out_off[q]] = o[q];
                 fence_proxy_async();
@@ -581,51 +612,34 @@ cudaError_t launch_dense_tc(void* amps, int qubits, const DenseOp& op, const flo
             lmask |= 1u << b;
             P.l_bits[nl++] = b;
         }
-    int r = 0;
-    bool seen_q = false;
-    while (r < qubits && ((qmask | lmask) >> r & 1u)) {
-        const bool is_q = (qmask >> r) & 1u;
-        if (!is_q && seen_q) break;
-        seen_q = seen_q || is_q;
-        ++r;
-    }
     for (int i = 0; i < 6; ++i) P.q_bits[i] = op.q[i];
-    P.cols_bits = c;
-    // one tensor-map box per tile where the tile's bit runs fit five dimensions: the staged tile
-    // is then in natural index order (unpadded), and so are its runs for bulk copies without an
-    // encoder; otherwise padded runs in which every column bit lies below every fused bit
+    P.tile_mask = qmask | lmask;
     int32_t rank = 0;
-    const bool natural = dense_tma_enabled() && (qmask | lmask) & 1u &&
-                         tile_map_dims(qmask | lmask, qubits, P.tma_lo, P.tma_len, P.tma_tile, &rank);
-    if (natural) {
-        r = 0;
-        while (r < qubits && ((qmask | lmask) >> r & 1u)) ++r;
-        if (encode_tile_map(&P.tmap, amps, QM_FP32, rank, P.tma_lo, P.tma_len, P.tma_tile)) P.tma_rank = rank;
+    if (dense_tma_enabled() && tile_map_dims(P.tile_mask, qubits, P.tma_lo, P.tma_len, P.tma_tile, &rank) &&
+        encode_tile_map(&P.tmap, amps, QM_FP32, rank, P.tma_lo, P.tma_len, P.tma_tile))
+        P.tma_rank = rank;
+    for (int b = 0, local = 0; b < qubits; ++b) {
+        if (!((P.tile_mask >> b) & 1u)) continue;
+        if (local >= 6)
+            for (int i = 0; i < 32; ++i)
+                if ((i >> (local - 6)) & 1) P.off[i] |= 1u << b;
+        ++local;
     }
-    P.run_bits = r;
-    P.copy_mask = (qmask | lmask) & ~((1u << r) - 1u);
-    P.copies = 1 << (kTcTileBits - r);
-    const int run_bytes = 8 << r;
-    P.stride = (1 << r) + (run_bytes >= 128 && !natural ? 2 : 0);
-    P.stage_elems = ((P.copies * P.stride * 8 + 127) / 128) * 16;
-    P.outer_mask = ((1u << qubits) - 1u) & ~(qmask | lmask);
+    P.outer_mask = ((1u << qubits) - 1u) & ~P.tile_mask;
     P.items = uint64_t(1) << (qubits - kTcTileBits);
-    const size_t stage_bytes = (size_t)P.stage_elems * 8;
-    P.stages = kOffStage + kTcMaxStages * stage_bytes <= kTcSmemMax ? kTcMaxStages : kTcMaxStages - 1;
-    const size_t smem = (size_t)kOffStage + (size_t)P.stages * stage_bytes;
-    if (smem > kTcSmemMax) return cudaErrorInvalidValue;
     std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_dense_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemMax);
+        attr = cudaFuncSetAttribute(k_dense_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
         if (attr == cudaSuccess)
-            attr = cudaFuncSetAttribute(k_dense_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemMax);
+            attr = cudaFuncSetAttribute(k_dense_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     });
     if (attr != cudaSuccess) return attr;
     const int grid = (int)std::min<uint64_t>(P.items, (uint64_t)std::max(1, sm_count));
+    const int threads = P.tma_rank ? kTcThreads : kTcCopyThreads;
     g_dense_tc_launches.fetch_add(1, std::memory_order_relaxed);
     if (lmask & 1u)
-        k_dense_tc<true><<<grid, kTcThreads, smem, st>>>(reinterpret_cast<float2*>(amps), P);
+        k_dense_tc<true><<<grid, threads, kTcSmem, st>>>(reinterpret_cast<float2*>(amps), P);
     else
-        k_dense_tc<false><<<grid, kTcThreads, smem, st>>>(reinterpret_cast<float2*>(amps), P);
+        k_dense_tc<false><<<grid, threads, kTcSmem, st>>>(reinterpret_cast<float2*>(amps), P);
     return cudaGetLastError();
 }
 
