@@ -1198,39 +1198,44 @@ int32_t validate_terms(const qm_pauli_term* terms, int32_t count, int qubits) {
     return QM_OK;
 }
 
-// Raw term sums and mass into host arrays (raw[count], *mass).  States of 9 or more qubits use
-// the tiled kernel (a few reads of the state for the whole term list); smaller ones run one
-// pass per distinct flip mask.
-int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, double* mass) {
+// Raw sums of the terms and the mass of a state of at least 9 qubits through the tiled kernel, whose
+// tiles hold flip masks of any width up to a tile; false when a mask spans more.
+bool tiled_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, int32_t* rc) {
     qm_context* ctx = st->ctx;
     TilePlan tp;
     std::string err;
-    if (st->qubits >= 9 && plan_tiles(st->qubits, st->precision, terms, count, tp, err)) {
+    if (!plan_tiles(st->qubits, st->precision, terms, count, tp, err)) return false;
+    auto run = [&]() -> int32_t {
         const size_t cells = (size_t)tp.rows_per_state * tp.columns;
-        int32_t rc = ensure_scratch(ctx, sizeof(double) * (cells + tp.columns));
-        if (rc) return rc;
-        rc = ensure_host_scratch(ctx, sizeof(double) * tp.columns);
-        if (rc) return rc;
+        int32_t r = ensure_scratch(ctx, sizeof(double) * (cells + tp.columns));
+        if (r) return r;
+        r = ensure_host_scratch(ctx, sizeof(double) * tp.columns);
+        if (r) return r;
         double* partial = static_cast<double*>(ctx->scratch);
         double* out = partial + cells;
         QM_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * cells, ctx->stream));
         for (const TilePass& p : tp.passes)
             QM_CUDA(launch_expect_tile(st->amps, st->qubits, st->precision, p, tp.terms.data(), 1, 0, partial,
                                        tp.columns, tp.rows_per_state, tp.mass_column, ctx->stream));
-        QM_CUDA(launch_finish_batched(partial, 1, tp.rows_per_state, tp.columns, out, ctx->stream));
+        QM_CUDA(launch_finish_sums(partial, tp.rows_per_state, tp.columns, out, ctx->stream));
         QM_CUDA(cudaMemcpyAsync(ctx->host_scratch, out, sizeof(double) * tp.columns, cudaMemcpyDeviceToHost,
                                 ctx->stream));
         QM_CUDA(cudaStreamSynchronize(ctx->stream));
         for (int32_t i = 0; i < count; ++i) raw[i] = ctx->host_scratch[i];
-        *mass = ctx->host_scratch[tp.mass_column];
         return QM_OK;
-    }
+    };
+    *rc = run();
+    return true;
+}
+
+// The same with the mass, one pass per distinct flip mask: any state and any mask.
+int32_t grouped_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, double* mass) {
+    qm_context* ctx = st->ctx;
     std::vector<DevPauli> dev((size_t)count);
     for (int32_t i = 0; i < count; ++i)
         dev[(size_t)i] = DevPauli{terms[i].flip_mask, terms[i].sign_mask, terms[i].y_count & 3, 0};
     const int columns = count + 1;
-    const int max_blocks = 148 * 4;
-    int32_t rc = ensure_scratch(ctx, sizeof(double) * ((size_t)max_blocks * columns + columns));
+    int32_t rc = ensure_scratch(ctx, sizeof(double) * ((size_t)kReduceBlocksMax * columns + columns));
     if (rc) return rc;
     rc = ensure_host_scratch(ctx, sizeof(double) * columns);
     if (rc) return rc;
@@ -1244,6 +1249,47 @@ int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t cou
     for (int32_t i = 0; i < count; ++i) raw[i] = ctx->host_scratch[i];
     *mass = ctx->host_scratch[count];
     return QM_OK;
+}
+
+// Raw term sums and mass into host arrays (raw[count], *mass).  States of 9 or more qubits take the
+// whole term list in a few reads of the state (qm_pauli_sum.cu), but for terms that flip more than
+// four qubits, which share the tiled kernel's passes; smaller states run one pass per flip mask.
+int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, double* mass) {
+    if (st->qubits < 9) return grouped_expectation(st, terms, count, raw, mass);
+    qm_context* ctx = st->ctx;
+    PauliSumPlan plan;
+    plan_pauli_sum(st->qubits, st->precision, terms, count, ctx->sm_count, plan);
+    const size_t program = pauli_sum_inline(plan) ? 0 : (plan.program.size() + 255) & ~size_t(255);
+    const size_t masses = (size_t)plan.parts * plan.tiles, cells = (size_t)plan.grid * plan.columns;
+    int32_t rc = ensure_scratch(ctx, program + sizeof(double) * (masses + cells + plan.columns));
+    if (rc) return rc;
+    rc = ensure_host_scratch(ctx, program + sizeof(double) * plan.columns);
+    if (rc) return rc;
+    double* tile_masses = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + program);
+    double* partials = tile_masses + masses;
+    double* out = partials + cells;
+    double* host = ctx->host_scratch + program / sizeof(double);
+    if (program) {
+        std::memcpy(ctx->host_scratch, plan.program.data(), plan.program.size());
+        QM_CUDA(cudaMemcpyAsync(ctx->scratch, ctx->host_scratch, plan.program.size(), cudaMemcpyHostToDevice, ctx->stream));
+    }
+    QM_CUDA(launch_pauli_sum(st->amps, st->precision, plan, program ? ctx->scratch : nullptr, tile_masses, partials,
+                             ctx->stream));
+    QM_CUDA(launch_finish_sums(partials, (int)plan.grid, plan.columns, out, ctx->stream));
+    QM_CUDA(cudaMemcpyAsync(host, out, sizeof(double) * plan.columns, cudaMemcpyDeviceToHost, ctx->stream));
+    QM_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int32_t i = 0; i < count; ++i) raw[i] = host[i];
+    *mass = host[count];
+    if (plan.wide.empty()) return QM_OK;
+    std::vector<qm_pauli_term> wide;
+    for (int i : plan.wide) wide.push_back(terms[i]);
+    std::vector<double> sums(wide.size());
+    if (!tiled_expectation(st, wide.data(), (int32_t)wide.size(), sums.data(), &rc)) {
+        double again = 0;
+        rc = grouped_expectation(st, wide.data(), (int32_t)wide.size(), sums.data(), &again);
+    }
+    for (size_t i = 0; rc == QM_OK && i < wide.size(); ++i) raw[plan.wide[i]] = sums[i];
+    return rc;
 }
 
 }  // namespace

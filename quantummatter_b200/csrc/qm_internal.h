@@ -315,6 +315,26 @@ cudaError_t launch_collapse(void* amps, int qubits, int precision, const SampleS
 cudaError_t launch_measure(void* amps, int qubits, int precision, uint64_t mask, SampleSummary* summary,
                            double* partials, cudaStream_t s);
 
+// ---------------------------------------------------------------- Pauli sums of one state (qm_pauli_sum.cu)
+// The passes of a term list over a state of at least 9 qubits: `program` is their device form, `wide`
+// the terms left out (they flip more than four qubits).  Terms that are zero for every state keep a
+// zero column.
+struct PauliSumPlan {
+    int qubits = 0, k = 0, passes = 0, diagonal_passes = 0, parts = 0, locals = 0, outers = 0, max_entries = 0, columns = 0;
+    uint32_t tiles = 0, grid = 0;
+    size_t at[6] = {};
+    bool zeros = false;  // some term is zero for every state: no kernel writes its column
+    std::vector<unsigned char> program;
+    std::vector<int> wide;
+};
+void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int count, int sm_count, PauliSumPlan& plan);
+// Whether the plan's program fits the kernels' parameters (launch_pauli_sum then takes no copy of it).
+bool pauli_sum_inline(const PauliSumPlan& plan);
+// Partial sums [grid][columns] of every term but the wide ones, the mass in the last column;
+// tile_masses holds parts * tiles doubles, `program` the plan's program in device memory or null.
+cudaError_t launch_pauli_sum(const void* amps, int precision, const PauliSumPlan& plan, const void* program,
+                             double* tile_masses, double* partials, cudaStream_t s);
+
 // ---------------------------------------------------------------- tiled expectation (qm_expect.cu)
 constexpr int kTileMaxTerms = 256;
 struct TileTerm {
