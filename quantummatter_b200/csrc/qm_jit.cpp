@@ -295,6 +295,10 @@ __device__ __forceinline__ void qm_arrive(u32 id, u32 n) { asm volatile("bar.arr
 #endif
 )SRC";
 
+// where code that the ops collect goes: run per state, and its variables
+constexpr const char* kPerState = "/*state*/";
+constexpr const char* kPerStateVars = "/*vars*/";
+
 struct Gen {
     std::ostringstream os;
     bool fp64;
@@ -506,15 +510,65 @@ struct Gen {
         close(n);
     }
 
+    // A complex factor of a diagonal group: two expressions, or exactly one.
+    struct Factor {
+        std::string re, im;
+        bool one = true;
+    };
+    Factor times(const Factor& a, const Factor& b) {
+        if (a.one) return b;
+        if (b.one) return a;
+        const std::string n = std::to_string(uid++);
+        os << "const " << T << " fr" << n << " = " << a.re << " * " << b.re << " - " << a.im << " * " << b.im << ", fi" << n
+           << " = " << a.re << " * " << b.im << " + " << a.im << " * " << b.re << ";\n";
+        return {"fr" + n, "fi" + n, false};
+    }
+
+    // Commuting diagonals as one phase per register.  Members on thread or outer bits fold into one
+    // factor u of the thread; members on register bits become a pair of factors per bit, and the
+    // phases are products of two small tables (four members: 42 complex products against 80 with one
+    // pass over the registers per member).  Table factors on thread bits do not depend on the tile:
+    // with `hoist` they are formed once per state.
+    std::ostringstream* hoist = nullptr;  // code run when a block turns to another state
+    std::string hoisted;                  // declarations of what it sets
     void group(int o, const std::vector<FusedOp>& ops, int first, int count) {
-        // register-bit phases per member; thread and outer phases folded into u
         bool any_u = false;
+        std::vector<int> early;
         for (int k = 0; k < count; ++k) {
             const FusedOp& m = ops[(size_t)(first + k)];
-            if (m.code == OP_DIAG && !(m.local >= 0 && reg_of_local(m.local) >= 0)) any_u = true;
+            if (m.code != OP_DIAG || (m.local >= 0 && reg_of_local(m.local) >= 0)) continue;
+            if (hoist && m.local >= 0 && (m.flags & kOpTable) && m.cmask_outer == 0) early.push_back(k);
+            else any_u = true;
+        }
+        std::string h;
+        auto fold_member = [&](std::ostringstream& out, const FusedOp& m, int om, const std::string& ur,
+                               const std::string& ui) {
+            const std::string c = coef_ptr(om, m);
+            if (m.local >= 0)
+                out << "{ const bool bt = ((base >> " << (int)m.local << ") & 1u) != 0u;\n";
+            else
+                out << "{ const bool bt = (outer & " << hexu(m.target_outer) << ") != 0u;\n";
+            out << "const " << T << " pr = (" << T << ")(bt ? " << c << "[6] : " << c << "[0]), pi = (" << T << ")(bt ? " << c
+                << "[7] : " << c << "[1]);\n";
+            out << "const " << T << " nr = " << ur << " * pr - " << ui << " * pi; " << ui << " = " << ur << " * pi + " << ui
+                << " * pr; " << ur << " = nr; }\n";
+        };
+        if (!early.empty()) {
+            h = std::to_string(uid++);
+            hoisted += std::string(T) + " hr" + h + " = (" + T + ")1, hi" + h + " = (" + T + ")0;\n";
+            *hoist << "{ const u32 base = " << base_expr() << "; hr" << h << " = (" << T << ")1; hi" << h << " = (" << T
+                   << ")0;\n";
+            for (int k : early) fold_member(*hoist, ops[(size_t)(first + k)], o + 1 + k, "hr" + h, "hi" + h);
+            *hoist << "}\n";
         }
         os << "{\n";
-        if (any_u) os << T << " ur = (" << T << ")1, ui = (" << T << ")0;\n";
+        if (any_u) {
+            if (early.empty())
+                os << T << " ur = (" << T << ")1, ui = (" << T << ")0;\n";
+            else
+                os << T << " ur = hr" << h << ", ui = hi" << h << ";\n";
+        }
+        Factor zero[R], on[R];
         for (int k = 0; k < count; ++k) {
             const FusedOp& m = ops[(size_t)(first + k)];
             const int om = o + 1 + k;
@@ -524,22 +578,43 @@ struct Gen {
             }
             const int M = m.local >= 0 ? reg_of_local(m.local) : -1;
             if (M >= 0) {
-                diag(om, m);
+                const std::string c = coef_ptr(om, m), n = std::to_string(uid++);
+                os << "const " << T << " zr" << n << " = (" << T << ")" << c << "[0], zi" << n << " = (" << T << ")" << c
+                   << "[1], or" << n << " = (" << T << ")" << c << "[6], oi" << n << " = (" << T << ")" << c << "[7];\n";
+                if (!(m.flags & 1)) zero[M] = times(zero[M], {"zr" + n, "zi" + n, false});
+                if (!(m.flags & 2)) on[M] = times(on[M], {"or" + n, "oi" + n, false});
                 continue;
             }
+            if (std::find(early.begin(), early.end(), k) != early.end()) continue;
             const int n = open_conditions(m.cmask_outer, 0);
-            const std::string c = coef_ptr(om, m);
-            if (m.local >= 0)
-                os << "{ const bool bt = ((base >> " << (int)m.local << ") & 1u) != 0u;\n";
-            else
-                os << "{ const bool bt = (outer & " << hexu(m.target_outer) << ") != 0u;\n";
-            os << "const " << T << " pr = (" << T << ")(bt ? " << c << "[6] : " << c << "[0]), pi = (" << T
-               << ")(bt ? " << c << "[7] : " << c << "[1]);\n";
-            os << "const " << T << " nr = ur * pr - ui * pi; ui = ur * pi + ui * pr; ur = nr; }\n";
+            fold_member(os, m, om, "ur", "ui");
             close(n);
         }
-        if (any_u)
-            for (int i = 0; i < NR; ++i) cmul_reg(i, "ur", "ui");
+        std::vector<int> bits;
+        for (int m = 0; m < R; ++m)
+            if (!zero[m].one || !on[m].one) bits.push_back(m);
+        // tables over the lower and the upper half of those bits; u goes into the upper one
+        Factor u;
+        if (any_u) u = {"ur", "ui", false};
+        else if (!early.empty()) u = {"hr" + h, "hi" + h, false};
+        const size_t half = bits.size() / 2;
+        std::vector<Factor> lo(1), hi(1, u);
+        for (size_t j = 0; j < bits.size(); ++j) {
+            std::vector<Factor>& table = j < half ? lo : hi;
+            std::vector<Factor> next;
+            for (const Factor& f : table) next.push_back(times(f, zero[bits[j]]));
+            for (const Factor& f : table) next.push_back(times(f, on[bits[j]]));
+            table.swap(next);
+        }
+        std::vector<Factor> phase;
+        for (const Factor& f : hi)
+            for (const Factor& l : lo) phase.push_back(times(l, f));
+        for (int i = 0; i < NR; ++i) {
+            size_t at = 0;
+            for (size_t j = 0; j < bits.size(); ++j)
+                if ((i >> bits[j]) & 1) at |= (size_t)1 << j;
+            if (!phase[at].one) cmul_reg(i, phase[at].re.c_str(), phase[at].im.c_str());
+        }
         os << "}\n";
     }
 
@@ -949,14 +1024,16 @@ struct Gen {
             os << "{\n";
             if (op.flags & kOpBranch) {
                 // noise branch: identity skipped, real diagonal as a scaling
-                os << "const double* c = " << c << ";\n";
-                os << "if (c[1] != 0.0 || c[3] != 0.0 || c[5] != 0.0 || c[7] != 0.0) {\n";
+                os << "const " << T << "* c = " << c << ";\n";
+                const std::string zero = std::string("(") + T + ")0", one = std::string("(") + T + ")1";
+                os << "if (c[1] != " << zero << " || c[3] != " << zero << " || c[5] != " << zero << " || c[7] != " << zero
+                   << ") {\n";
                 load_coef("c", false);
                 pairs_matrix(M, rm, false);
-                os << "} else if (c[2] != 0.0 || c[4] != 0.0) {\n";
+                os << "} else if (c[2] != " << zero << " || c[4] != " << zero << ") {\n";
                 load_coef("c", true);
                 pairs_matrix(M, rm, true);
-                os << "} else if (!(c[0] == 1.0 && c[6] == 1.0)) {\n";
+                os << "} else if (!(c[0] == " << one << " && c[6] == " << one << ")) {\n";
                 os << "const " << T << " s0 = (" << T << ")c[0], s1 = (" << T << ")c[6];\n";
                 for (int i = 0; i < NR; ++i) {
                     const char* s = ((i >> M) & 1) ? "s1" : "s0";
@@ -1364,7 +1441,7 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     if (late) os << "V* ptile = tile;\n";
     if (hist) os << "double* hacc = reinterpret_cast<double*>(smem_raw + " << tiles * tile_bytes << ");\n";
     os << "FusedOp* prog = reinterpret_cast<FusedOp*>(smem_raw + " << tiles * tile_bytes + hist_bytes << ");\n";
-    os << "double* table = reinterpret_cast<double*>(smem_raw + " << (tiles * tile_bytes + hist_bytes + prog_bytes)
+    os << g.T << "* table = reinterpret_cast<" << g.T << "*>(smem_raw + " << (tiles * tile_bytes + hist_bytes + prog_bytes)
        << ");\n";
     os << (teams ? "const u32 t = threadIdx.x & " + hexu((uint32_t)nt - 1u) + ";\n" : "const u32 t = threadIdx.x;\n");
     os << "{ const uint2* src = reinterpret_cast<const uint2*>(P.ops); uint2* dst = reinterpret_cast<uint2*>(prog);\n"
@@ -1400,6 +1477,10 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     const char* next_item = teams ? "item + 2 * (long long)gridDim.x" : "item + gridDim.x";
     prefetch(teams ? "(long long)blockIdx.x + (long long)team * gridDim.x" : "(long long)blockIdx.x");
     os << "int current = -1;\n";
+    // complex64 has the registers to keep what depends on the state alone
+    std::ostringstream per_state;
+    if (tabled && !fp64) g.hoist = &per_state;
+    if (tabled) os << kPerStateVars;
     if (hist) {
         os << "for (long long u = blockIdx.x; u < total / " << chunk << "; u += gridDim.x) {\n";
         os << "for (int i = t; i < " << warps * hist_bins << "; i += " << nt << ") hacc[i] = 0.0;\n";
@@ -1410,6 +1491,9 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
         os << "for (long long k2 = 0; (long long)blockIdx.x + k2 * gridDim.x < total; k2 += 2) {\n";
         os << "const long long item = (long long)blockIdx.x + (k2 + (long long)team) * gridDim.x;\n";
         os << "if (item >= total) { for (int j = 0; j < " << segs << "; ++j) { " << acquire << release << "} continue; }\n";
+    } else if (tabled) {
+        // consecutive tiles: a block stays with a state, whose row it stages once (18 qubits: 64 tiles)
+        os << "for (long long item = total * blockIdx.x / gridDim.x; item < total * (blockIdx.x + 1ll) / gridDim.x; ++item) {\n";
     } else {
         os << "for (long long item = blockIdx.x; item < total; item += gridDim.x) {\n";
     }
@@ -1418,7 +1502,7 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     os << g.bar;
     if (tabled)
         os << "if (P.table_slots > 0 && b != current) { const double* row = P.table + (u64)b * P.table_stride;\n"
-           << "  for (int i = t; i < 8 * P.table_slots; i += " << nt << ") table[i] = __ldg(row + i); __syncthreads(); }\n";
+           << "  for (int i = t; i < 8 * P.table_slots; i += " << nt << ") table[i] = (" << g.T << ")__ldg(row + i); __syncthreads();\n" << kPerState << "}\n";
     os << "current = b;\n";
     os << "V* __restrict__ s = s0 + (u64)b * P.state_stride;\n";
     os << "const u32 outer = qm_deposit(cta, P.outer_mask);\n";
@@ -1587,6 +1671,12 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     // the constants travel as a kernel parameter (at most 32764 bytes with the launch record)
     if (g.aux.size() > kMaxAuxValues + 1000) return out;
     out.src = hd.str() + os.str();
+    auto place = [&](const char* mark, const std::string& code) {
+        const size_t at = out.src.find(mark);
+        if (at != std::string::npos) out.src.replace(at, std::strlen(mark), code);
+    };
+    place(kPerStateVars, g.hoisted);
+    place(kPerState, per_state.str());
     out.tiles = tiles;
     out.teams = teams ? 2 : 1;
     out.hist_bins = hist_bins;
