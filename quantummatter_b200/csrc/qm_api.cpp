@@ -295,7 +295,15 @@ int32_t build_plan(qm_context* ctx, int32_t qubits, int32_t precision, const qm_
     std::vector<qm_gate> list(gates, gates + count);
     std::string err;
     if (width == 0) width = ctx->fusion_width;
-    if (!plan_fused(list, qubits, precision, width, plan, err)) return fail(QM_E_ARG, "planner: " + err);
+    // States too small for a fused block, and one-shot executions of up to kSmallQubits qubits, run
+    // their gates in one block (one block of interpreted passes takes twice as long, and planning them
+    // 0.1 ms for a hundred gates).  Plans of nine qubits and more run compiled passes.
+    plan.small = width == 0 && qubits <= (transient ? kSmallQubits : 8);
+    if (!plan_fused(list, qubits, precision, plan.small ? 1 : width, plan, err)) return fail(QM_E_ARG, "planner: " + err);
+    if (plan.small) {
+        plan.launches = (int32_t)((plan.gates.size() + kSmallGates - 1) / kSmallGates);
+        plan.planned_bytes = 2ll * (precision == QM_FP32 ? 8 : 16) << qubits;
+    }
     // one-shot executions of large states run the compiled passes already built for the same
     // structures; they never wait for a compilation.  Below 26 qubits a pass takes well under a
     // millisecond, about what generating the plan's sources for the lookup costs on the host,
@@ -319,7 +327,15 @@ int32_t run_plan(qm_context* ctx, const Plan& plan, void* amps, const volatile i
         }
         return QM_OK;
     };
-    if (plan.width == 1) {
+    if (plan.small) {
+        const int total = (int)plan.gates.size();
+        for (int g = 0; g < total; g += kSmallGates) {
+            QM_CUDA(launch_small(amps, plan.qubits, plan.precision, plan.gates.data() + g,
+                                 std::min(kSmallGates, total - g), ctx->stream));
+            int32_t rc = chunk_boundary();
+            if (rc) return rc;
+        }
+    } else if (plan.width == 1) {
         for (const DevGate& g : plan.gates) {
             QM_CUDA(launch_gate(amps, plan.qubits, plan.precision, g, ctx->stream));
             int32_t rc = chunk_boundary();

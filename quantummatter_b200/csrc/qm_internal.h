@@ -164,6 +164,7 @@ struct Plan {
     bool start_zero = false;
     bool zero_fused = false;
     bool borrowed = false;          // d_ops belongs to a context buffer
+    bool small = false;             // the gates run in one block, kSmallGates a launch (launch_small)
     std::vector<DenseOp> dense;         // dense fused gates (widths 2..6)
     std::vector<double> dense_matrices; // their transposed unitaries, (re, im) pairs
     double* d_dense = nullptr;          // device copy of dense_matrices
@@ -265,6 +266,10 @@ FusedLaunch fused_launch_params(int qubits, const FusedPass& p, const FusedOp* d
 void jit_prepare(Plan& plan);
 void jit_lookup(Plan& plan);  // compiled kernels already in the cache only (no compilation)
 cudaError_t launch_plan_pass(const Plan& plan, size_t pass, void* amps, const FusedBatch* batch, cudaStream_t s);
+// Up to kSmallGates gates in order on a state of at most kSmallQubits qubits, in one launch (they
+// travel as its parameter).
+constexpr int kSmallQubits = 11, kSmallGates = 384;
+cudaError_t launch_small(void* amps, int qubits, int precision, const DevGate* gates, int count, cudaStream_t s);
 cudaError_t launch_reset(void* amps, int qubits, int precision, cudaStream_t s);
 cudaError_t launch_convert_from_f64(void* dst_f32, const double* src_f64, int64_t n, cudaStream_t s);
 cudaError_t launch_convert_to_f64(double* dst_f64, const void* src_f32, int64_t n, cudaStream_t s);

@@ -135,6 +135,127 @@ cudaError_t launch_gate_t(void* amps, int qubits, const DevGate& g, cudaStream_t
     return cudaGetLastError();
 }
 
+// Up to kSmallGates gates on a state of at most kSmallQubits qubits in one launch: the state sits in
+// one block's shared memory and the gates run one after another, a pair of amplitudes per thread (up
+// to four).  Such a state fills a fraction of one SM, so the serial chain bounds it: 0.2 to 0.4 us a
+// gate (mask and coefficient loads, amplitude loads, four dependent multiply-adds, stores, a barrier).
+// The barrier is of the warp while targets are among the lowest six qubits, whose pairs keep to 64
+// amplitudes per warp (and 64 more per further pair).  Device time of a brick of depth 26, against one
+// launch per gate (8 qubits: 1198 to 62 us for 299 gates) and passes of 16 amplitudes per thread, two
+// warps or four in all (10 qubits: 221 to 104 us for 377 gates; 11: 249 to 178).
+constexpr int kSmallThreads = 256;
+static_assert(1 << (kSmallQubits - 1) <= 4 * kSmallThreads, "at most four pairs per thread");
+
+struct SmallGate {
+    int32_t kernel, target;
+    uint32_t control, swap;
+    double c[8];
+};
+template <int N>
+struct SmallProgram {
+    int32_t qubits, count;
+    SmallGate gate[N];
+};
+
+// The gates travel as a kernel parameter: the constant cache feeds their masks and coefficients, and
+// shared memory only the amplitudes.  At most eight warps, with PAIRS pairs per thread, since every
+// warp loads every gate.
+template <typename T, int N, int PAIRS>
+__global__ void __launch_bounds__(kSmallThreads) k_small(typename Vec2<T>::type* __restrict__ s,
+                                                         const __grid_constant__ SmallProgram<N> P) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using V = typename Vec2<T>::type;
+    V* state = reinterpret_cast<V*>(smem);
+    const uint32_t t = threadIdx.x, nt = blockDim.x, pairs = 1u << (P.qubits - 1);
+    for (uint32_t i = t; i < 2 * pairs; i += nt) state[i] = s[i];
+    __syncthreads();
+    bool wide = false;  // the previous gate left its warp's amplitudes
+    SmallGate next = P.gate[0];
+    for (int k = 0; k < P.count; ++k) {
+        const SmallGate g = next;
+        next = P.gate[min(k + 1, P.count - 1)];  // asked for a gate ahead: it is a constant-cache miss
+        const bool spans = g.target >= 6 || g.swap >= 64u;
+        if (wide || spans) __syncthreads();
+        else __syncwarp();
+        wide = spans;
+        const uint32_t need = g.control | g.swap;
+        uint32_t f[PAIRS], o[PAIRS];
+        bool on[PAIRS];
+        Cx<T> x[PAIRS], y[PAIRS];
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) {
+            f[j] = insert_zero(t + kSmallThreads * j, g.target);
+            on[j] = t < pairs && (f[j] & need) == need;
+            // a swap trades target 0 and swap bit 1 for target 1 and swap bit 0
+            o[j] = (f[j] ^ g.swap) | (1u << g.target);
+            if (on[j]) {
+                x[j] = load_amp<T>(state, f[j]);
+                y[j] = load_amp<T>(state, o[j]);
+            }
+        }
+        if (g.kernel == QM_KERNEL_MATRIX) {
+#pragma unroll
+            for (int j = 0; j < PAIRS; ++j) {
+                if (!on[j]) continue;
+                store_amp<T>(state, f[j], cmac2<T>((T)g.c[0], (T)g.c[1], x[j], (T)g.c[2], (T)g.c[3], y[j]));
+                store_amp<T>(state, o[j], cmac2<T>((T)g.c[4], (T)g.c[5], x[j], (T)g.c[6], (T)g.c[7], y[j]));
+            }
+        } else if (g.kernel == QM_KERNEL_HADAMARD) {
+            const T h = (T)g.c[0];
+#pragma unroll
+            for (int j = 0; j < PAIRS; ++j) {
+                if (!on[j]) continue;
+                store_amp<T>(state, f[j], Cx<T>{h * x[j].re + h * y[j].re, h * x[j].im + h * y[j].im});
+                store_amp<T>(state, o[j], Cx<T>{h * x[j].re - h * y[j].re, h * x[j].im - h * y[j].im});
+            }
+        } else if (g.kernel == QM_KERNEL_DIAGONAL) {
+            const bool a_one = g.c[0] == 1.0 && g.c[1] == 0.0, d_one = g.c[6] == 1.0 && g.c[7] == 0.0;
+#pragma unroll
+            for (int j = 0; j < PAIRS; ++j) {
+                if (on[j] && !a_one) store_amp<T>(state, f[j], cmul<T>((T)g.c[0], (T)g.c[1], x[j]));
+                if (on[j] && !d_one) store_amp<T>(state, o[j], cmul<T>((T)g.c[6], (T)g.c[7], y[j]));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < PAIRS; ++j) {
+                if (!on[j]) continue;
+                store_amp<T>(state, f[j], y[j]);
+                store_amp<T>(state, o[j], x[j]);
+            }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < 2 * pairs; i += nt) s[i] = state[i];
+}
+
+template <typename T, int N>
+cudaError_t launch_small_n(void* amps, int qubits, const DevGate* gates, int count, cudaStream_t st) {
+    SmallProgram<N> P;
+    P.qubits = qubits;
+    P.count = count;
+    for (int k = 0; k < count; ++k) {
+        const DevGate& g = gates[k];
+        SmallGate& o = P.gate[k];
+        o.kernel = g.kernel;
+        o.target = g.target;
+        o.control = g.control_mask;
+        o.swap = g.swap_bit;
+        for (int i = 0; i < 2; ++i) {
+            o.c[i] = g.a[i];
+            o.c[2 + i] = g.b[i];
+            o.c[4 + i] = g.c[i];
+            o.c[6 + i] = g.d[i];
+        }
+    }
+    using V = typename Vec2<T>::type;
+    const int pairs = 1 << (qubits - 1), threads = std::min(kSmallThreads, std::max(32, pairs));
+    const size_t smem = sizeof(V) << qubits;
+    if (pairs <= kSmallThreads) k_small<T, N, 1><<<1, threads, smem, st>>>(static_cast<V*>(amps), P);
+    else if (pairs == 2 * kSmallThreads) k_small<T, N, 2><<<1, threads, smem, st>>>(static_cast<V*>(amps), P);
+    else k_small<T, N, 4><<<1, threads, smem, st>>>(static_cast<V*>(amps), P);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- state utilities
 
 template <typename T>
@@ -671,6 +792,15 @@ __global__ void k_collapse(typename Vec2<T>::type* s, uint64_t n, const SampleSu
 
 cudaError_t launch_gate(void* amps, int qubits, int precision, const DevGate& g, cudaStream_t s) {
     return precision == QM_FP32 ? launch_gate_t<float>(amps, qubits, g, s) : launch_gate_t<double>(amps, qubits, g, s);
+}
+
+cudaError_t launch_small(void* amps, int qubits, int precision, const DevGate* gates, int count, cudaStream_t st) {
+    if (qubits < 1 || qubits > kSmallQubits || count < 0 || count > kSmallGates) return cudaErrorInvalidValue;
+    if (precision == QM_FP32)
+        return count <= 48 ? launch_small_n<float, 48>(amps, qubits, gates, count, st)
+                           : launch_small_n<float, kSmallGates>(amps, qubits, gates, count, st);
+    return count <= 48 ? launch_small_n<double, 48>(amps, qubits, gates, count, st)
+                       : launch_small_n<double, kSmallGates>(amps, qubits, gates, count, st);
 }
 
 cudaError_t launch_reset(void* amps, int qubits, int precision, cudaStream_t st) {
