@@ -12,6 +12,8 @@ from dataclasses import dataclass
 from enum import IntEnum
 from typing import Iterable, Sequence
 
+import numpy as np
+
 from .errors import ArgumentError, ArgumentOutOfRangeError
 
 
@@ -205,24 +207,28 @@ class QuantumCircuit:
         return self._add(GateKind.Toffoli, target, first, second=second)
 
 
+_OPERATION = np.dtype([("kind", "<i4"), ("target", "<i4"), ("control", "<i4"), ("second_control", "<i4"),
+                       ("angle", "<f8"), ("unitary", "<f8", 8)])  # qm_operation
+
+
 def operations_array(ops: Iterable[GateOperation]):
-    """Packs GateOperation records into a ctypes qm_operation array."""
+    """Packs GateOperation records into a ctypes qm_operation array, a column at a time."""
     from ._lib import Operation
     ops = list(ops)
-    arr = (Operation * max(1, len(ops)))()
-    for i, o in enumerate(ops):
-        r = arr[i]
-        r.kind = int(o.Kind)
-        r.target = o.Target
-        r.control = o.Control
-        r.second_control = o.SecondControl
-        r.angle = o.Angle
-        if o.Unitary is not None:
-            u = o.Unitary
-            vals = (u.M00.real, u.M00.imag, u.M01.real, u.M01.imag, u.M10.real, u.M10.imag, u.M11.real, u.M11.imag)
-            for j, v in enumerate(vals):
-                r.unitary[j] = v
-    return arr, len(ops)
+    n = len(ops)
+    arr = (Operation * max(1, n))()
+    if n:
+        rec = np.frombuffer(arr, dtype=_OPERATION)
+        rec["kind"] = [int(o.Kind) for o in ops]
+        rec["target"] = [o.Target for o in ops]
+        rec["control"] = [o.Control for o in ops]
+        rec["second_control"] = [o.SecondControl for o in ops]
+        rec["angle"] = [o.Angle for o in ops]
+        at = [i for i, o in enumerate(ops) if o.Unitary is not None]
+        if at:
+            entries = [v for i in at for u in (ops[i].Unitary,) for v in (u.M00, u.M01, u.M10, u.M11)]
+            rec["unitary"][at] = np.array(entries, dtype=np.complex128).view(np.float64).reshape(-1, 8)
+    return arr, n
 
 
 def prepare(circuit: QuantumCircuit):

@@ -40,6 +40,27 @@ int32_t cuda_fail(cudaError_t err, const char* what) {
 
 using namespace qm;
 
+cudaError_t pool_alloc(qm_context* ctx, void** out, size_t bytes) {
+    if (bytes > kPoolKeep) return cudaMalloc(out, bytes);
+    if (!ctx->pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
+        uint64_t keep = kPoolKeep;
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaMallocFromPoolAsync(out, bytes, ctx->pool, ctx->stream);
+}
+
+void pool_free(qm_context* ctx, void* pointer, size_t bytes) {
+    if (!pointer) return;
+    if (bytes > kPoolKeep) cudaFree(pointer);  // waits for the work that uses it
+    else cudaFreeAsync(pointer, ctx->stream);
+}
+
 namespace {
 
 constexpr int64_t kDefaultBudget = 512ll * 1024 * 1024;
@@ -454,6 +475,7 @@ extern "C" int32_t qm_context_create(const qm_options* options, qm_context** out
     cudaDeviceProp prop;
     QM_CUDA(cudaGetDeviceProperties(&prop, ctx->device));
     ctx->sm_count = prop.multiProcessorCount;
+    ctx->total_memory = (int64_t)prop.totalGlobalMem;
     QM_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     QM_CUDA(cudaEventCreate(&ctx->ev_start));
     QM_CUDA(cudaEventCreate(&ctx->ev_stop));
@@ -471,6 +493,8 @@ extern "C" int32_t qm_context_destroy(qm_context* ctx) {
         if (ctx->host_scratch) cudaFreeHost(ctx->host_scratch);
         if (ctx->staging) cudaFree(ctx->staging);
         if (ctx->program) cudaFree(ctx->program);
+        if (ctx->pinned) cudaFreeHost(ctx->pinned);
+        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
         release_bounce(ctx);
         if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
         if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
@@ -545,10 +569,8 @@ extern "C" int32_t qm_execute_host(qm_context* ctx, int32_t qubits, const qm_ope
     if (ctx->disposed) return fail(QM_E_DISPOSED, "context disposed");
     if (cancelled(cancel)) return fail(QM_E_CANCELLED, "operation cancelled");
     const int64_t bytes = 16 * length;
-    size_t free_b = 0, total_b = 0;
     QM_CUDA(cudaSetDevice(ctx->device));
-    QM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (bytes > ctx->device_budget || bytes > (int64_t)total_b || bytes > ctx->staging_budget)
+    if (bytes > ctx->device_budget || bytes > ctx->total_memory || bytes > ctx->staging_budget)
         return fail(QM_E_BUDGET, "CUDA state exceeds the device or host staging memory budget.");
     int32_t rc = validate_operations(ops, count, qubits);
     if (rc) return rc;
@@ -727,8 +749,14 @@ extern "C" int32_t qm_state_create(qm_context* ctx, int32_t qubits, int32_t prec
     st->qubits = qubits;
     st->precision = precision;
     st->bytes = bytes;
-    QM_CUDA(cudaMalloc(&st->amps, (size_t)bytes));
-    cudaError_t e = launch_reset(st->amps, qubits, precision, ctx->stream);
+    cudaError_t e = cudaMalloc(&st->amps, (size_t)bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->pool) {  // what the pool keeps may be what is missing
+        cudaGetLastError();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMalloc(&st->amps, (size_t)bytes);
+    }
+    QM_CUDA(e);
+    e = launch_reset(st->amps, qubits, precision, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(st->amps);

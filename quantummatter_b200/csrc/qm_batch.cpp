@@ -149,12 +149,12 @@ int32_t check_batch(qm_batch* b) {
 }
 
 template <typename T>
-int32_t grow(T*& ptr, size_t& have, size_t need) {
+int32_t grow(qm_context* ctx, T*& ptr, size_t& have, size_t need) {
     if (have >= need) return QM_OK;
-    if (ptr) cudaFree(ptr);
+    pool_free(ctx, ptr, have);
     ptr = nullptr;
     have = 0;
-    QM_CUDA(cudaMalloc(reinterpret_cast<void**>(&ptr), need));
+    QM_CUDA(pool_alloc(ctx, reinterpret_cast<void**>(&ptr), need));
     have = need;
     return QM_OK;
 }
@@ -171,9 +171,9 @@ int32_t enqueue_plan(qm_batch* b, const Plan& plan, int states, const double* d_
 // and the mass in the last column).
 int32_t enqueue_tiles(qm_batch* b, const TilePlan& tp, int states, cudaStream_t st) {
     const size_t partial = sizeof(double) * (size_t)states * tp.rows_per_state * tp.columns;
-    int32_t rc = grow(b->partials, b->partial_bytes, partial);
+    int32_t rc = grow(b->ctx, b->partials, b->partial_bytes, partial);
     if (rc) return rc;
-    rc = grow(b->out, b->out_bytes, sizeof(double) * (size_t)states * tp.columns);
+    rc = grow(b->ctx, b->out, b->out_bytes, sizeof(double) * (size_t)states * tp.columns);
     if (rc) return rc;
     QM_CUDA(enqueue_tile_expectation(b->amps, b->qubits, b->precision, tp, states, b->partials, b->out, st));
     return QM_OK;
@@ -215,11 +215,11 @@ extern "C" int32_t qm_batch_create(qm_context* ctx, int32_t qubits, int32_t prec
     b->precision = precision;
     b->capacity = capacity;
     b->state_bytes = state_bytes;
-    QM_CUDA(cudaMalloc(&b->amps, (size_t)bytes));
+    QM_CUDA(pool_alloc(ctx, &b->amps, (size_t)bytes));
     cudaError_t e = launch_reset_batched(b->amps, qubits, precision, capacity, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        cudaFree(b->amps);
+        pool_free(ctx, b->amps, (size_t)bytes);
         return cuda_fail(e, "qm_batch_create");
     }
     ctx->device_in_use += bytes;
@@ -233,10 +233,11 @@ extern "C" int32_t qm_batch_destroy(qm_batch* b) {
         std::lock_guard<std::recursive_mutex> lock(b->ctx->mu);
         cudaSetDevice(b->ctx->device);
         cudaStreamSynchronize(b->ctx->stream);
-        cudaFree(b->amps);
-        if (b->table) cudaFree(b->table);
-        if (b->partials) cudaFree(b->partials);
-        if (b->out) cudaFree(b->out);
+        pool_free(b->ctx, b->amps, (size_t)(b->state_bytes * b->capacity));
+        pool_free(b->ctx, b->table, b->table_bytes);
+        pool_free(b->ctx, b->partials, b->partial_bytes);
+        pool_free(b->ctx, b->out, b->out_bytes);
+        cudaStreamSynchronize(b->ctx->stream);  // beyond kPoolKeep the pool gives memory back here
         b->ctx->device_in_use -= b->state_bytes * b->capacity;
     }
     delete b;
@@ -316,7 +317,7 @@ extern "C" int32_t qm_batch_execute(qm_batch* b, int32_t states, const qm_gate* 
     if (rc) return rc;
     const size_t tbytes = sizeof(double) * (size_t)states * slot_count * 8;
     if (tbytes) {
-        rc = grow(b->table, b->table_bytes, tbytes);
+        rc = grow(ctx, b->table, b->table_bytes, tbytes);
         if (rc) return rc;
         QM_CUDA(cudaMemcpyAsync(b->table, table, tbytes, cudaMemcpyHostToDevice, ctx->stream));
     }
@@ -438,6 +439,9 @@ struct VqeProblem {
     Plan plan;
     TilePlan tp;
     qm_batch* batch = nullptr;
+    qm_context* owner = nullptr;  // of the plan's program on the device
+    void* program = nullptr;
+    size_t program_bytes = 0;
     int B = 0;
     double* h_table[2] = {nullptr, nullptr};
     double* h_out[2] = {nullptr, nullptr};
@@ -453,10 +457,10 @@ struct VqeProblem {
     VqeProblem(const VqeProblem&) = delete;
     VqeProblem& operator=(const VqeProblem&) = delete;
     ~VqeProblem() {
-        plan_release(plan);
-        for (int i = 0; i < 2; ++i) {
-            if (h_table[i]) cudaFreeHost(h_table[i]);
-            if (h_out[i]) cudaFreeHost(h_out[i]);
+        if (own_stream && stream) cudaStreamSynchronize(stream);  // work of a wave that failed to join
+        if (program) {
+            std::lock_guard<std::recursive_mutex> lock(owner->mu);
+            pool_free(owner, program, program_bytes);
         }
         if (batch) qm_batch_destroy(batch);
         if (own_stream && stream) cudaStreamDestroy(stream);
@@ -530,8 +534,14 @@ struct VqeProblem {
             return fail(QM_E_ARG, "planner: " + err);
         plan.start_zero = true;  // every circuit starts from |0...0>
         jit_prepare(plan);       // one structure for every circuit of every wave
-        int32_t rc = plan_upload(plan, ctx->stream);
-        if (rc) return rc;
+        if (!plan.ops.empty()) {
+            program_bytes = plan.ops.size() * sizeof(FusedOp);
+            QM_CUDA(pool_alloc(ctx, &program, program_bytes));
+            plan.d_ops = static_cast<FusedOp*>(program);
+            plan.borrowed = true;
+            owner = ctx;
+            QM_CUDA(cudaMemcpyAsync(program, plan.ops.data(), program_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        }
         if (!plan_tiles(exec_qubits, precision, terms, term_count, tp, err)) return fail(QM_E_ARG, err);
         jit_prepare_tiles(tp, exec_qubits, precision);  // one term list for every circuit of every wave
         const double half_pi = M_PI / 2;
@@ -550,7 +560,7 @@ struct VqeProblem {
     }
 
     // The device batch: as many states as `bytes` allow (at least one) and a wave has use for, its
-    // table, tile partials and pinned host buffers, all at full size before any capture.
+    // table and tile partials, all at full size before any capture.
     int32_t allocate(qm_context* ctx, int64_t bytes, int64_t resident) {
         int64_t cap = std::min<int64_t>({circuits, 65535, bytes / std::max<int64_t>(state_bytes(), 1), 8192});
         if (cap < 1) return fail(QM_E_BUDGET, "a single state exceeds the context's device memory budget");
@@ -561,17 +571,24 @@ struct VqeProblem {
         if (rc) return rc;
         B = (int)cap;
         const size_t table_doubles = (size_t)B * slot_count * 8;
-        rc = grow(batch->table, batch->table_bytes, sizeof(double) * table_doubles);
+        rc = grow(ctx, batch->table, batch->table_bytes, sizeof(double) * table_doubles);
         if (rc) return rc;
-        rc = grow(batch->partials, batch->partial_bytes, sizeof(double) * (size_t)B * tp.rows_per_state * tp.columns);
+        rc = grow(ctx, batch->partials, batch->partial_bytes, sizeof(double) * (size_t)B * tp.rows_per_state * tp.columns);
         if (rc) return rc;
-        rc = grow(batch->out, batch->out_bytes, sizeof(double) * (size_t)B * tp.columns);
+        rc = grow(ctx, batch->out, batch->out_bytes, sizeof(double) * (size_t)B * tp.columns);
         if (rc) return rc;
-        for (int i = 0; i < 2; ++i) {
-            QM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_table[i]), sizeof(double) * table_doubles));
-            QM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_out[i]), sizeof(double) * (size_t)B * tp.columns));
-        }
         return QM_OK;
+    }
+
+    // This problem's page-locked transfer buffers, from `at` on; returns what follows them.
+    double* host_buffers(double* at) {
+        for (int i = 0; i < 2; ++i) {
+            h_table[i] = at;
+            at += (size_t)B * slot_count * 8;
+            h_out[i] = at;
+            at += (size_t)B * tp.columns;
+        }
+        return at;
     }
 
     void fill_table(int buf, int64_t first, int count) {
@@ -706,6 +723,29 @@ int32_t run_problems(qm_context* ctx, std::vector<std::unique_ptr<VqeProblem>>& 
         int32_t rc = p->allocate(ctx, share, (int64_t)((double)kResidentBytes * part));
         if (rc) return rc;
     }
+    // transfer buffers of all problems in the context's page-locked block
+    size_t pinned = 0;
+    for (auto& p : problems)
+        pinned += 2 * sizeof(double) * ((size_t)p->B * p->slot_count * 8 + (size_t)p->B * p->tp.columns);
+    if (ctx->pinned_bytes < pinned) {
+        if (ctx->pinned) cudaFreeHost(ctx->pinned);
+        ctx->pinned = nullptr;
+        ctx->pinned_bytes = 0;
+        QM_CUDA(cudaMallocHost(&ctx->pinned, pinned));
+        ctx->pinned_bytes = pinned;
+    }
+    struct PinnedGuard {  // a large block is not kept
+        qm_context* ctx;
+        ~PinnedGuard() {
+            if (ctx->pinned_bytes <= kPinnedKeep) return;
+            cudaStreamSynchronize(ctx->stream);
+            cudaFreeHost(ctx->pinned);
+            ctx->pinned = nullptr;
+            ctx->pinned_bytes = 0;
+        }
+    } pinned_guard{ctx};
+    double* host = static_cast<double*>(ctx->pinned);
+    for (auto& p : problems) host = p->host_buffers(host);
     const bool multi = problems.size() > 1;
     cudaStream_t main = ctx->stream;
     for (auto& p : problems) {

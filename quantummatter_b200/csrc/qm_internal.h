@@ -478,6 +478,13 @@ struct qm_context {
     size_t scratch_bytes = 0;
     double* host_scratch = nullptr;   // pinned, for small downloads
     size_t host_scratch_bytes = 0;
+    // device memory of batch calls, allocated and freed in the stream's order: a call's buffers stay
+    // with the context up to kPoolKeep bytes, the rest goes back to the device (pool_alloc)
+    cudaMemPool_t pool = nullptr;
+    // page-locked host memory of a batch call's transfers, kept up to kPinnedKeep bytes
+    void* pinned = nullptr;
+    size_t pinned_bytes = 0;
+    int64_t total_memory = 0;
     // device buffer of the host-buffer entry points (qm_execute_host, qm_noise_apply_host)
     void* staging = nullptr;
     size_t staging_bytes = 0;
@@ -488,6 +495,13 @@ struct qm_context {
     void* bounce[2] = {nullptr, nullptr};
     cudaEvent_t bounce_done[2] = {nullptr, nullptr};
 };
+// Device memory of a batch call on the context's stream, the same `bytes` to free it; callers hold the
+// context's lock.  Up to kPoolKeep bytes come from the context's pool; larger ones are plain
+// allocations (1.6 GB through the pool is mapped anew on each call: 10 ms more per trajectory run).
+constexpr uint64_t kPoolKeep = 128ull << 20;
+constexpr size_t kPinnedKeep = 32u << 20;
+cudaError_t pool_alloc(qm_context* ctx, void** out, size_t bytes);
+void pool_free(qm_context* ctx, void* pointer, size_t bytes);
 // Whole-state copies with a caller's host buffer on the context's stream (qm_transfer.cpp):
 // host_to_device returns once the host buffer has been read (the device copy may still be in
 // flight on the stream); device_to_host returns once the host buffer holds the data.

@@ -1784,14 +1784,16 @@ namespace {
 bool compile_all(const std::vector<Generated>& gen) {
     std::vector<size_t> todo;
     {
+        // sources not compiled yet, each once
         std::unordered_map<std::string, size_t> first;
+        std::lock_guard<std::mutex> lock(g_cache_mu);
         for (size_t i = 0; i < gen.size(); ++i)
-            if (first.emplace(gen[i].src, i).second) todo.push_back(i);
+            if (!g_cache.count(gen[i].src) && first.emplace(gen[i].src, i).second) todo.push_back(i);
     }
     int device = 0;
     cudaGetDevice(&device);
     std::atomic<size_t> next{0};
-    const size_t workers = std::max<size_t>(1, std::min<size_t>(todo.size(), std::thread::hardware_concurrency()));
+    const size_t workers = std::min<size_t>(todo.size(), std::max(1u, std::thread::hardware_concurrency()));
     std::vector<std::thread> pool;
     for (size_t w = 0; w < workers; ++w)
         pool.emplace_back([&]() {

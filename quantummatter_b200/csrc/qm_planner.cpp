@@ -30,8 +30,16 @@ namespace qm {
 
 namespace {
 
+// A gate as the passes move and rename it: its coefficients stay where the caller has them.
+struct PlanGate {
+    int32_t kernel, target;
+    uint32_t control_mask;
+    int32_t swap_control;
+    const double *a, *b, *c, *d;
+};
+
 struct GInfo {
-    qm_gate g;
+    PlanGate g;
     int32_t slot;    // batch-table coefficient slot, -1 for constant coefficients
     bool diag;
     uint32_t touch;  // every qubit the gate reads
@@ -42,24 +50,23 @@ struct GInfo {
 
 inline int popc(uint32_t x) { return __builtin_popcount(x); }
 
-GInfo classify(const qm_gate& g) {
-    GInfo gi{};
-    gi.g = g;
-    gi.slot = -1;
+// the roles of a gate's qubits
+void set_masks(GInfo& gi) {
+    const PlanGate& g = gi.g;
     uint32_t tb = 1u << g.target;
     uint32_t sb = g.kernel == QM_KERNEL_SWAP ? (1u << g.swap_control) : 0u;
     gi.touch = tb | sb | g.control_mask;
-    if (g.kernel == QM_KERNEL_DIAGONAL) {
-        gi.diag = true;
-        gi.xmask = 0;
-        gi.zmask = gi.touch;
-        gi.need = 0;
-    } else {
-        gi.diag = false;
-        gi.xmask = tb | sb;
-        gi.zmask = g.control_mask;
-        gi.need = tb | sb;
-    }
+    gi.diag = g.kernel == QM_KERNEL_DIAGONAL;
+    gi.xmask = gi.diag ? 0u : tb | sb;
+    gi.zmask = gi.diag ? gi.touch : g.control_mask;
+    gi.need = gi.xmask;
+}
+
+GInfo classify(const qm_gate& g, int32_t slot) {
+    GInfo gi{};
+    gi.g = PlanGate{g.kernel, g.target, g.control_mask, g.swap_control, g.a, g.b, g.c, g.d};
+    gi.slot = slot;
+    set_masks(gi);
     return gi;
 }
 
@@ -67,16 +74,13 @@ inline bool blocked(const GInfo& g, uint32_t bx, uint32_t bz) { return (g.touch 
 
 // a gate's qubits renamed by a permutation of the index bits
 void remap_gate(GInfo& gi, const int* perm) {
-    qm_gate g = gi.g;
+    PlanGate& g = gi.g;
     g.target = perm[g.target];
     uint32_t cm = 0;
-    for (int q = 0; q < 32; ++q)
-        if (g.control_mask & (1u << q)) cm |= 1u << perm[q];
+    for (uint32_t m = g.control_mask; m; m &= m - 1) cm |= 1u << perm[__builtin_ctz(m)];
     g.control_mask = cm;
     if (g.kernel == QM_KERNEL_SWAP) g.swap_control = perm[g.swap_control];
-    const int32_t slot = gi.slot;
-    gi = classify(g);
-    gi.slot = slot;
+    set_masks(gi);
 }
 
 inline bool is_exact(const double* v, double re, double im) { return v[0] == re && v[1] == im; }
@@ -187,9 +191,7 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
             error = "a noise branch is an uncontrolled matrix placeholder";
             return false;
         }
-        GInfo info = classify(g);
-        info.slot = slot;
-        remaining.push_back(info);
+        remaining.push_back(classify(g, slot));
     }
 
     // Low qubits always in the block: 8 complex128 or 16 complex64 = one 128-byte run.
@@ -238,8 +240,7 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
             pass.op_begin = (int32_t)plan.ops.size();
             auto to_local = [&](uint32_t global) {
                 uint32_t l = 0;
-                for (int q = 0; q < qubits; ++q)
-                    if (global & (1u << q)) l |= 1u << local_of[q];
+                for (uint32_t m = global; m; m &= m - 1) l |= 1u << local_of[__builtin_ctz(m)];
                 return l;
             };
 
@@ -365,12 +366,12 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
                     group_qubits = 0;
                 };
                 for (const GInfo& gi : stage_gates[si]) {
-                    const qm_gate& g = gi.g;
+                    const PlanGate& g = gi.g;
                     FusedOp op{};
                     op.reg = op.reg2 = -1;
                     op.local = -1;
-                    for (int q = 0; q < qubits; ++q) {
-                        if (!(g.control_mask & (1u << q))) continue;
+                    for (uint32_t m = g.control_mask; m; m &= m - 1) {
+                        const int q = __builtin_ctz(m);
                         if (local_of[q] >= 0) op.cmask_local |= (uint16_t)(1u << local_of[q]);
                         else op.cmask_outer |= 1u << q;
                     }
@@ -661,15 +662,24 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
             place(Q);
         } else if (relabel) {
             // the low_bits bits of Q whose qubits let the next pass absorb the most gates
+            // (several hundred choices are tried, so the masks are read from a compact list)
+            struct Masks {
+                uint32_t touch, xmask, zmask, need;
+            };
+            std::vector<Masks> masks;
+            masks.reserve(rest.size());
+            for (const GInfo& g : rest) masks.push_back(Masks{g.touch, g.xmask, g.zmask, g.need});
             auto absorbable = [&](uint32_t start) {
                 uint32_t QQ = start, cx = 0, cz = 0;
-                int c = 0;
-                for (const GInfo& g : rest) {
+                int c = 0, room = k - popc(start);
+                for (const Masks& g : masks) {
                     if (c >= kMaxPassGates || cx == all_qubits) break;
-                    if (!blocked(g, cx, cz)) {
-                        const uint32_t nq = QQ | g.need;
-                        if (popc(nq) <= k) {
-                            QQ = nq;
+                    if (!((g.touch & cx) | (g.xmask & cz))) {
+                        const uint32_t add = g.need & ~QQ;  // a target, or both operands of a swap
+                        const int bits = (add != 0) + ((add & (add - 1)) != 0);
+                        if (bits <= room) {
+                            QQ |= add;
+                            room -= bits;
                             ++c;
                             continue;
                         }

@@ -266,18 +266,19 @@ struct Buffers {
     cudaStream_t stream;
     qm_context* ctx;
     int64_t accounted = 0;
-    std::vector<void*> ptrs;
+    std::vector<std::pair<void*, size_t>> ptrs;
     Buffers(qm_context* c) : stream(c->stream), ctx(c) {}
     ~Buffers() {
+        for (auto& p : ptrs) pool_free(ctx, p.first, p.second);
         cudaStreamSynchronize(stream);
-        for (void* p : ptrs) cudaFree(p);
         ctx->device_in_use -= accounted;
     }
     template <typename T>
     int32_t get(T*& out, size_t bytes) {
         void* p = nullptr;
-        QM_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-        ptrs.push_back(p);
+        bytes = std::max<size_t>(bytes, 16);
+        QM_CUDA(pool_alloc(ctx, &p, bytes));
+        ptrs.push_back({p, bytes});
         out = static_cast<T*>(p);
         return QM_OK;
     }
@@ -381,8 +382,18 @@ extern "C" int32_t qm_trajectories_run(qm_context* ctx, int32_t qubits, int32_t 
         // epilogue of its last pass when that pass compiles
         if (s.group >= 0 && !s.plan.passes.empty()) s.plan.hist_mask = P.groups[(size_t)s.group];
         jit_prepare(s.plan);  // layers repeat: most segments share compiled passes
-        rc = plan_upload(s.plan, st);
-        if (rc) return rc;
+    }
+    // the segments' programs in one buffer
+    std::vector<FusedOp> ops;
+    for (const Segment& s : P.segments) ops.insert(ops.end(), s.plan.ops.begin(), s.plan.ops.end());
+    FusedOp* d_ops = nullptr;
+    if ((rc = buf.get(d_ops, sizeof(FusedOp) * ops.size()))) return rc;
+    if (!ops.empty())
+        QM_CUDA(cudaMemcpyAsync(d_ops, ops.data(), sizeof(FusedOp) * ops.size(), cudaMemcpyHostToDevice, st));
+    for (Segment& s : P.segments) {
+        s.plan.d_ops = d_ops;
+        s.plan.borrowed = true;
+        d_ops += s.plan.ops.size();
     }
 
     const double margin = precision == QM_FP32 ? 1e-5 : 1e-12;
