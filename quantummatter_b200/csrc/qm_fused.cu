@@ -34,9 +34,16 @@ namespace {
 constexpr int R = kRegBits;
 constexpr int NR = 1 << R;
 
+// An op's a, b, c, d in the state's precision: the kernel converts the program's and the table row's
+// coefficients once, when it stages them.
+template <typename T>
 struct Coef {
-    double v[8];
+    T v[8];
 };
+template <typename T>
+__device__ __forceinline__ const T* op_coef(const FusedOp& op) {
+    return reinterpret_cast<const T*>(op.coef);
+}
 
 // Shared-memory slot of local index j: the low row bits are XORed with a fold of the
 // higher bits, so that the 8 (complex128) or 16 (complex64) lanes of one shared-memory
@@ -100,10 +107,10 @@ __device__ __forceinline__ uint32_t control_pattern(const Layout& L, uint32_t cm
 }
 
 template <typename T, int M, bool REAL, bool CTRL>
-__device__ __forceinline__ void op_matrix(Cx<T> (&a)[NR], const FusedOp& op, const Coef& c, const Layout& L) {
-    const T ar = (T)c.v[0], br = (T)c.v[2], cr = (T)c.v[4], dr = (T)c.v[6];
-    const T ai = REAL ? (T)0 : (T)c.v[1], bi = REAL ? (T)0 : (T)c.v[3];
-    const T ci = REAL ? (T)0 : (T)c.v[5], di = REAL ? (T)0 : (T)c.v[7];
+__device__ __forceinline__ void op_matrix(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L) {
+    const T ar = c.v[0], br = c.v[2], cr = c.v[4], dr = c.v[6];
+    const T ai = REAL ? (T)0 : c.v[1], bi = REAL ? (T)0 : c.v[3];
+    const T ci = REAL ? (T)0 : c.v[5], di = REAL ? (T)0 : c.v[7];
     const uint32_t pat = CTRL ? control_pattern(L, op.cmask_local) : 0u;
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
@@ -122,7 +129,7 @@ __device__ __forceinline__ void op_matrix(Cx<T> (&a)[NR], const FusedOp& op, con
 }
 
 template <typename T, bool REAL, bool CTRL>
-__device__ __forceinline__ void op_matrix_any(Cx<T> (&a)[NR], const FusedOp& op, const Coef& c, const Layout& L) {
+__device__ __forceinline__ void op_matrix_any(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L) {
     switch (op.reg) {
     case 0: op_matrix<T, 0, REAL, CTRL>(a, op, c, L); break;
     case 1: op_matrix<T, 1, REAL, CTRL>(a, op, c, L); break;
@@ -149,7 +156,7 @@ __device__ __forceinline__ void op_scale(Cx<T> (&a)[NR], T s0, T s1) {
 // coefficients are mostly the identity (no Pauli error) or a real diagonal (a damping without
 // a jump, a Z error); the test is uniform across the CTA, which works on one state.
 template <typename T>
-__device__ __forceinline__ void op_branch(Cx<T> (&a)[NR], const FusedOp& op, const Coef& c, const Layout& L) {
+__device__ __forceinline__ void op_branch(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L) {
     const bool real = c.v[1] == 0 && c.v[3] == 0 && c.v[5] == 0 && c.v[7] == 0;
     if (!real) {
         op_matrix_any<T, false, false>(a, op, c, L);
@@ -160,7 +167,7 @@ __device__ __forceinline__ void op_branch(Cx<T> (&a)[NR], const FusedOp& op, con
         return;
     }
     if (c.v[0] == 1 && c.v[6] == 1) return;
-    const T s0 = (T)c.v[0], s1 = (T)c.v[6];
+    const T s0 = c.v[0], s1 = c.v[6];
     switch (op.reg) {
     case 0: op_scale<T, 0>(a, s0, s1); break;
     case 1: op_scale<T, 1>(a, s0, s1); break;
@@ -281,8 +288,8 @@ __device__ __forceinline__ void slots(const Layout& L, uint32_t (&s)[NR]) {
 // Diagonal whose target bit is a register bit M: the phase of each register is known at
 // compile time.
 template <typename T, int M>
-__device__ __forceinline__ void op_diag_reg(Cx<T> (&a)[NR], const FusedOp& op, const Coef& c, const Layout& L) {
-    const T ar = (T)c.v[0], ai = (T)c.v[1], dr = (T)c.v[6], di = (T)c.v[7];
+__device__ __forceinline__ void op_diag_reg(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L) {
+    const T ar = c.v[0], ai = c.v[1], dr = c.v[6], di = c.v[7];
     const bool a_one = op.flags & 1, d_one = op.flags & 2;
     const uint32_t pat = control_pattern(L, op.cmask_local);
 #pragma unroll
@@ -297,9 +304,9 @@ __device__ __forceinline__ void op_diag_reg(Cx<T> (&a)[NR], const FusedOp& op, c
 }
 
 template <typename T>
-__device__ __forceinline__ void op_diag(Cx<T> (&a)[NR], const FusedOp& op, const Coef& c, const Layout& L,
+__device__ __forceinline__ void op_diag(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L,
                                         uint32_t outer) {
-    const T ar = (T)c.v[0], ai = (T)c.v[1], dr = (T)c.v[6], di = (T)c.v[7];
+    const T ar = c.v[0], ai = c.v[1], dr = c.v[6], di = c.v[7];
     const bool a_one = op.flags & 1, d_one = op.flags & 2;
     const uint32_t cm = op.cmask_local;
     const int lt = op.local;
@@ -352,14 +359,16 @@ __device__ __forceinline__ Cx<T> cmulc(Cx<T> x, Cx<T> y) {
     return Cx<T>{x.re * y.re - x.im * y.im, x.re * y.im + x.im * y.re};
 }
 
-// A group of commuting diagonals applied as one phase per register.  Every member's factor
-// splits by where its qubits sit: outside the block or on a thread bit it is one value for
-// the whole thread (folded into u); on a register bit m it is a pair (zero-phase, one-phase)
-// multiplied into (az[m], on[m]); a negate on register bits flips the sign of the registers
-// whose index has those bits (a 16-bit pattern).  Then phase[i] = u * prod_m (i_m ? on : az)
-// is built as a product tree and applied once.
+// A group of commuting diagonals applied as one phase per register.  Every member's factor splits by
+// where its qubits sit: outside the block or on a thread bit it is one value for the whole thread
+// (folded into u); on a register bit m it is a pair (zero-phase, one-phase) multiplied into (az[m],
+// on[m]); a negate on register bits flips the sign of the registers whose index has those bits (a
+// 16-bit pattern).  Controls outside the registers decide whether the thread takes part; one control
+// on a register bit takes the one-phase of that bit.  What needs two register bits goes over the
+// registers directly (op_diag; it commutes).  Then phase[i] = u * prod_m (i_m ? on : az) is built as a
+// product tree and applied once.
 template <typename T>
-__device__ __forceinline__ void op_diag_group(Cx<T> (&a)[NR], const FusedOp* members, int count, const double* table,
+__device__ __forceinline__ void op_diag_group(Cx<T> (&a)[NR], const FusedOp* members, int count, const T* table,
                                               const Layout& L, uint32_t outer) {
     Cx<T> u{(T)1, (T)0};
     Cx<T> az[R], on[R];
@@ -373,30 +382,100 @@ __device__ __forceinline__ void op_diag_group(Cx<T> (&a)[NR], const FusedOp* mem
     uint32_t regmask = 0;
 #pragma unroll
     for (int m = 0; m < R; ++m) regmask |= L.pm[m];
+    // Phases on one register bit (a ladder's target) multiply up in `acc` before they go to that bit.
+    uint32_t held = 0;
+    Cx<T> acc{(T)1, (T)0};
+    auto release = [&]() {
+#pragma unroll
+        for (int m = 0; m < R; ++m)
+            if (L.pm[m] == held) on[m] = cmulc<T>(on[m], acc);
+        acc = Cx<T>{(T)1, (T)0};
+    };
     for (int k = 0; k < count; ++k) {
         const FusedOp& op = members[k];
-        if ((outer & op.cmask_outer) != op.cmask_outer) continue;
-        if (op.code == OP_NEGATE) {
-            negate ^= control_pattern(L, op.cmask_local);
+        // the record's first 24 bytes in three loads
+        const uint2* words = reinterpret_cast<const uint2*>(&op);
+        const uint2 w0 = words[0], w1 = words[1], w2 = words[2];
+        const uint32_t code = w0.x & 0xffu, flags = w1.x >> 16;
+        uint32_t local = w1.x & 0xffffu, out_bits = w1.y;
+        if ((outer & out_bits) != out_bits) continue;
+        if (code == OP_NEGATE) {
+            negate ^= control_pattern(L, local);
             continue;
         }
+        const int lt = (int)(int8_t)(w0.x >> 24);
+        const uint32_t target = lt >= 0 ? 1u << lt : 0u;
+        const T* src = (flags & kOpTable) ? table + 8 * (size_t)w2.y : op_coef<T>(op);
+        const Cx<T> pd{src[6], src[7]};
         phased = true;
-        // uncontrolled single-qubit diagonal
-        const double* src = (op.flags & kOpTable) ? table + 8 * (size_t)op.reserved : op.coef;
-        const Cx<T> pa{(T)src[0], (T)src[1]}, pd{(T)src[6], (T)src[7]};
-        const int lt = op.local;
-        if (lt >= 0 && (regmask & (1u << lt))) {
+        if (flags & 1) {
+            // a phase where the target and every control are one: all its qubits are alike
+            out_bits = w2.x;
+            local |= target;
+            if ((outer & out_bits) != out_bits) continue;
+            const uint32_t regs = local & regmask, thread = local & ~regmask;
+            const bool takes = (L.base & thread) == thread;
+            const Cx<T> p{takes ? pd.re : (T)1, takes ? pd.im : (T)0};
+            if (regs == 0) {
+                u = cmulc<T>(u, p);
+            } else if ((regs & (regs - 1)) == 0) {
+                if (regs != held) {
+                    release();
+                    held = regs;
+                }
+                acc = cmulc<T>(acc, p);
+            } else {
+                // two register bits: a quarter of the registers (more bits: the pairs' pattern)
+                bool pair = false;
+#pragma unroll
+                for (int m1 = 0; m1 < R; ++m1)
+#pragma unroll
+                    for (int m2 = m1 + 1; m2 < R; ++m2)
+                        if (regs == (L.pm[m1] | L.pm[m2])) {
+                            pair = true;
+#pragma unroll
+                            for (int i = 0; i < NR; ++i)
+                                if (((i >> m1) & 1) && ((i >> m2) & 1)) a[i] = cmul<T>(p.re, p.im, a[i]);
+                        }
+                if (!pair) {
+                    const uint32_t pat = control_pattern(L, regs);
+#pragma unroll
+                    for (int i = 0; i < NR; ++i)
+                        if ((pat >> i) & 1u) a[i] = cmul<T>(p.re, p.im, a[i]);
+                }
+            }
+            continue;
+        }
+        const Cx<T> pa{src[0], src[1]};
+        const uint32_t creg = local & regmask, cthread = local & ~regmask;
+        if (creg && ((target & regmask) || (creg & (creg - 1)))) {
+            Coef<T> c;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) c.v[i] = src[i];
+            op_diag<T>(a, op, c, L, outer);
+            continue;
+        }
+        if ((L.base & cthread) != cthread) continue;
+        if (target & regmask) {
 #pragma unroll
             for (int m = 0; m < R; ++m)
-                if (L.pm[m] == (1u << lt)) {
+                if (L.pm[m] == target) {
                     az[m] = cmulc<T>(az[m], pa);
                     on[m] = cmulc<T>(on[m], pd);
                 }
             continue;
         }
-        const bool bit = lt < 0 ? (outer & op.target_outer) != 0 : ((L.base >> lt) & 1u) != 0;
-        u = cmulc<T>(u, bit ? pd : pa);
+        const bool bit = lt < 0 ? (outer & w2.x) != 0 : (L.base & target) != 0;
+        const Cx<T> p = bit ? pd : pa;
+        if (creg) {
+#pragma unroll
+            for (int m = 0; m < R; ++m)
+                if (L.pm[m] == creg) on[m] = cmulc<T>(on[m], p);
+        } else {
+            u = cmulc<T>(u, p);
+        }
     }
+    release();
     if (!phased) {  // only CZ / Z members: signs
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
@@ -429,10 +508,15 @@ __device__ __forceinline__ void op_diag_group(Cx<T> (&a)[NR], const FusedOp* mem
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const Cx<T> p = cmulc<T>(lo[i & ((1 << LB) - 1)], hi[i >> LB]);
-        Cx<T> v = cmulc<T>(p, a[i]);
-        const bool neg = (negate >> i) & 1u;
-        a[i].re = neg ? -v.re : v.re;
-        a[i].im = neg ? -v.im : v.im;
+        a[i] = cmulc<T>(p, a[i]);
+    }
+    if (negate) {
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const bool neg = (negate >> i) & 1u;
+            a[i].re = neg ? -a[i].re : a[i].re;
+            a[i].im = neg ? -a[i].im : a[i].im;
+        }
     }
 }
 
@@ -453,13 +537,25 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* tile = reinterpret_cast<V*>(smem_raw);
     FusedOp* prog = reinterpret_cast<FusedOp*>(smem_raw + tile_bytes<T, K>());
-    double* table = reinterpret_cast<double*>(smem_raw + tile_bytes<T, K>() + program_bytes(P.op_count));
+    T* table = reinterpret_cast<T*>(smem_raw + tile_bytes<T, K>() + program_bytes(P.op_count));
     const uint32_t t = threadIdx.x;
     {
         const uint2* src = reinterpret_cast<const uint2*>(P.ops);
         uint2* dst = reinterpret_cast<uint2*>(prog);
         const int words = P.op_count * (int)(sizeof(FusedOp) / sizeof(uint2));
         for (int i = t; i < words; i += blockDim.x) dst[i] = __ldg(src + i);
+    }
+    if (sizeof(T) == 4) {  // coefficients to single precision, in place
+        __syncthreads();
+        for (int i = t; i < P.op_count; i += blockDim.x) {
+            if (prog[i].code == OP_STAGE || prog[i].code == OP_DIAG_GROUP) continue;
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = prog[i].coef[k];
+            T* c = reinterpret_cast<T*>(prog[i].coef);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[k] = (T)v[k];
+        }
     }
     const int64_t total = (int64_t)P.states << P.cta_shift;
     const uint32_t cta_mask = (1u << P.cta_shift) - 1u;
@@ -470,7 +566,7 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
         __syncthreads();  // program staged / previous block's exchanges finished
         if (P.table_slots > 0 && b != current) {
             const double* row = P.table + (size_t)b * P.table_stride;
-            for (int i = t; i < 8 * P.table_slots; i += blockDim.x) table[i] = __ldg(row + i);
+            for (int i = t; i < 8 * P.table_slots; i += blockDim.x) table[i] = (T)__ldg(row + i);
             __syncthreads();
         }
         current = b;
@@ -537,11 +633,23 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
                 o += count;
                 continue;
             }
+            if (code == OP_DIAG) {
+                // a run of diagonals, controlled or not (a Fourier transform's phase ladders): one
+                // phase per register.  25-qubit complex128 transform: 8.6 ms with a pass over the
+                // registers per phase, 4.8 ms so.
+                int count = 1;
+                while (o + count < P.op_count && prog[o + count].code == OP_DIAG) ++count;
+                if (count > 1) {
+                    op_diag_group<T>(a, prog + o, count, table, L, outer);
+                    o += count - 1;
+                    continue;
+                }
+            }
             if ((outer & op.cmask_outer) != op.cmask_outer) continue;
             const bool ctrl = op.cmask_local != 0;
-            Coef c;
+            Coef<T> c;
             if (code == OP_MATRIX || code == OP_MATRIX_REAL || code == OP_DIAG) {
-                const double* src = (op.flags & kOpTable) ? table + 8 * (size_t)op.reserved : op.coef;
+                const T* src = (op.flags & kOpTable) ? table + 8 * (size_t)op.reserved : op_coef<T>(op);
                 // only the entries the op kind reads
                 if (code == OP_MATRIX) {
 #pragma unroll
@@ -550,14 +658,14 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
 #pragma unroll
                     for (int k = 0; k < 8; k += 2) {
                         c.v[k] = src[k];
-                        c.v[k + 1] = 0.0;
+                        c.v[k + 1] = (T)0;
                     }
                 } else {
                     c.v[0] = src[0];
                     c.v[1] = src[1];
                     c.v[6] = src[6];
                     c.v[7] = src[7];
-                    c.v[2] = c.v[3] = c.v[4] = c.v[5] = 0.0;
+                    c.v[2] = c.v[3] = c.v[4] = c.v[5] = (T)0;
                 }
             }
             switch (code) {
