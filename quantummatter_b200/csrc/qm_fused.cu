@@ -128,6 +128,43 @@ __device__ __forceinline__ void op_matrix(Cx<T> (&a)[NR], const FusedOp& op, con
     }
 }
 
+// A matrix with a 1 in its first column (kOpRotation): [[1, -t lambda], [t, lambda]], or with B
+// [[t, -lambda], [1, t lambda]].  The coefficients are t, B and lambda: 8 multiply-adds per pair
+// against 16.
+template <typename T, int M>
+__device__ __forceinline__ void op_rotation(Cx<T> (&a)[NR], T t, bool form_b, T lr, T li) {
+    // both forms as x' = p x - q w, y' = q x + p w with one of p, q equal to 1
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        if ((i >> M) & 1) continue;
+        const int k = i | (1 << M);
+        const Cx<T> x = a[i], w = cmul<T>(lr, li, a[k]);
+        if (form_b) {
+            a[i] = Cx<T>{t * x.re - w.re, t * x.im - w.im};
+            a[k] = Cx<T>{x.re + t * w.re, x.im + t * w.im};
+        } else {
+            a[i] = Cx<T>{x.re - t * w.re, x.im - t * w.im};
+            a[k] = Cx<T>{t * x.re + w.re, t * x.im + w.im};
+        }
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void op_rotation_any(Cx<T> (&a)[NR], int reg, const T* c) {
+    const T t = c[0], lr = c[2], li = c[3];
+    const bool form_b = c[1] != (T)0;
+    switch (reg) {
+    case 0: op_rotation<T, 0>(a, t, form_b, lr, li); break;
+    case 1: op_rotation<T, 1>(a, t, form_b, lr, li); break;
+#if QM_REG_BITS > 3
+    case 2: op_rotation<T, 2>(a, t, form_b, lr, li); break;
+    default: op_rotation<T, 3>(a, t, form_b, lr, li); break;
+#else
+    default: op_rotation<T, 2>(a, t, form_b, lr, li); break;
+#endif
+    }
+}
+
 template <typename T, bool REAL, bool CTRL>
 __device__ __forceinline__ void op_matrix_any(Cx<T> (&a)[NR], const FusedOp& op, const Coef<T>& c, const Layout& L) {
     switch (op.reg) {
@@ -545,17 +582,29 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
         const int words = P.op_count * (int)(sizeof(FusedOp) / sizeof(uint2));
         for (int i = t; i < words; i += blockDim.x) dst[i] = __ldg(src + i);
     }
-    if (sizeof(T) == 4) {  // coefficients to single precision, in place
-        __syncthreads();
-        for (int i = t; i < P.op_count; i += blockDim.x) {
-            if (prog[i].code == OP_STAGE || prog[i].code == OP_DIAG_GROUP) continue;
-            double v[8];
+    // coefficients in the state's precision, in place, and the matrices that run as rotations
+    __syncthreads();
+    for (int i = t; i < P.op_count; i += blockDim.x) {
+        if (prog[i].code == OP_STAGE || prog[i].code == OP_DIAG_GROUP) continue;
+        double v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = prog[i].coef[k];
-            T* c = reinterpret_cast<T*>(prog[i].coef);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) c[k] = (T)v[k];
+        for (int k = 0; k < 8; ++k) v[k] = prog[i].coef[k];
+        if (prog[i].code == OP_MATRIX && !(prog[i].flags & kOpTable) && prog[i].cmask_local == 0 && v[1] == 0.0 &&
+            v[5] == 0.0 && (v[0] == 1.0 || v[4] == 1.0)) {
+            const bool form_b = v[0] != 1.0;
+            const double tv = form_b ? v[0] : v[4], lr = form_b ? -v[2] : v[6], li = form_b ? -v[3] : v[7];
+            const double er = form_b ? v[6] - tv * lr : v[2] + tv * lr, ei = form_b ? v[7] - tv * li : v[3] + tv * li;
+            if (fabs(er) + fabs(ei) <= 4e-16 * (fabs(lr) + fabs(li))) {
+                prog[i].flags |= kOpRotation;
+                v[0] = tv;
+                v[1] = form_b ? 1.0 : 0.0;
+                v[2] = lr;
+                v[3] = li;
+            }
         }
+        T* c = reinterpret_cast<T*>(prog[i].coef);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = (T)v[k];
     }
     const int64_t total = (int64_t)P.states << P.cta_shift;
     const uint32_t cta_mask = (1u << P.cta_shift) - 1u;
@@ -646,6 +695,10 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
                 }
             }
             if ((outer & op.cmask_outer) != op.cmask_outer) continue;
+            if (op.flags & kOpRotation) {
+                op_rotation_any<T>(a, op.reg, op_coef<T>(op));
+                continue;
+            }
             const bool ctrl = op.cmask_local != 0;
             Coef<T> c;
             if (code == OP_MATRIX || code == OP_MATRIX_REAL || code == OP_DIAG) {

@@ -61,6 +61,7 @@ constexpr int kMaxPassOps = 256;    // ops per pass: the program (88 B per op) i
 constexpr int kMaxPassGates = 120;  // gates absorbed per pass (stage changes add at most gates + 2)
 
 constexpr uint16_t kOpTable = 4;    // FusedOp::flags: coefficients come from the batch's table
+constexpr uint16_t kOpRotation = 16;  // set by the interpreting kernel on its own copy of a program: see k_fused
 constexpr uint16_t kOpBranch = 8;   // FusedOp::flags: a table op realising a noise branch; the kernel
                                     // skips identities and applies real diagonals as scalings
 // A coefficient slot passed to plan_fused with this bit set marks a noise-branch op (kOpBranch).
@@ -183,8 +184,12 @@ void plan_release(Plan& plan);
 // Builds the fused schedule (qm_planner.cpp).  Returns false with a message on error.
 // slots (optional, one per gate): batch-table coefficient slot of each gate, -1 for gates
 // whose coefficients are the same for every state of a batch.
+// relabel: whether plans that write qubits to other index bits are tried (several hundred choices
+// per pass on the host).
 bool plan_fused(const std::vector<qm_gate>& gates, int qubits, int precision, int width, Plan& plan,
-                std::string& error, const std::vector<int32_t>* slots = nullptr);
+                std::string& error, const std::vector<int32_t>* slots = nullptr, bool relabel = true);
+// The same circuit in the form the interpreting kernel runs cheapest.
+std::vector<qm_gate> one_shot_gates(const std::vector<qm_gate>& gates, int precision);
 int default_block_qubits(int qubits, int precision);
 // Dense fused gates of at most `width` (1..6) qubits (qm_dense.cpp).
 bool plan_dense(const std::vector<qm_gate>& gates, int qubits, int precision, int width, Plan& plan,

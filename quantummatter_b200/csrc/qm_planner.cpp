@@ -19,6 +19,7 @@
 // Such a plan is kept only when it needs fewer passes than the plain one.
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -820,14 +821,138 @@ std::vector<qm_gate> cnots_as_cz(const std::vector<qm_gate>& gates) {
     return out;
 }
 
+// The gates of a one-shot execution, whose passes the interpreting kernel runs: every uncontrolled
+// 2x2 matrix is U = g diag(1, phi) R diag(1, lambda) with R = m [[1, -t], [t, 1]] when |u00| >= |u10|,
+// else m [[t, -1], [1, t]].  phi moves forward to the next matrix on its qubit (diagonals and controls
+// commute with it), uncontrolled diagonals with it, and g m to a later matrix, so what is left to run is
+// R / m times diag(1, lambda), recognised by the kernel by its 1: 8 multiply-adds per pair against 16.
+// A qubit's last matrix before a gate that phi cannot pass stays whole; one takes the scale up whenever
+// it falls below `least` (unscaled amplitudes grow by its inverse) and the last one takes all of it.
+std::vector<qm_gate> real_columns(const std::vector<qm_gate>& gates, int precision) {
+    using cd = std::complex<double>;
+    const double least = precision == QM_FP32 ? 1e-6 : 1e-60;
+    const long n = (long)gates.size();
+    auto plain = [](const qm_gate& g) {
+        return (g.kernel == QM_KERNEL_MATRIX || g.kernel == QM_KERNEL_HADAMARD) && g.control_mask == 0;
+    };
+    // the next gate that acts non-diagonally on each gate's target, and the last plain matrix of all
+    std::vector<long> next((size_t)n, -1);
+    long last_plain = -1;
+    {
+        long seen[32];
+        std::fill(seen, seen + 32, -1L);
+        for (long i = n; i-- > 0;) {
+            const qm_gate& g = gates[(size_t)i];
+            if (g.kernel == QM_KERNEL_IDENTITY) continue;
+            next[(size_t)i] = seen[g.target];
+            if (last_plain < 0 && plain(g)) last_plain = i;
+            if (g.kernel == QM_KERNEL_DIAGONAL) continue;
+            seen[g.target] = i;
+            if (g.kernel == QM_KERNEL_SWAP) seen[g.swap_control] = i;
+        }
+    }
+    std::vector<qm_gate> out;
+    out.reserve(gates.size());
+    cd phase[32], scale(1.0, 0.0);
+    std::fill(phase, phase + 32, cd(1.0, 0.0));
+    auto set = [](double* dst, cd v) {
+        dst[0] = v.real();
+        dst[1] = v.imag();
+    };
+    auto flush = [&](int q) {
+        if (phase[q] == cd(1.0, 0.0)) return;
+        qm_gate d{};
+        d.kernel = QM_KERNEL_DIAGONAL;
+        d.target = q;
+        d.swap_control = -1;
+        set(d.a, cd(1.0, 0.0));
+        set(d.d, phase[q]);
+        out.push_back(d);
+        phase[q] = cd(1.0, 0.0);
+    };
+    for (long i = 0; i < n; ++i) {
+        const qm_gate& g = gates[(size_t)i];
+        if (g.kernel == QM_KERNEL_IDENTITY) continue;
+        const int q = g.target;
+        if (!plain(g)) {
+            // phi passes diagonals and controls, and takes up an uncontrolled diagonal; anything else on
+            // its qubit has it applied first
+            if (g.kernel != QM_KERNEL_DIAGONAL) {
+                flush(q);
+                if (g.kernel == QM_KERNEL_SWAP) flush(g.swap_control);
+            } else if (g.control_mask == 0 && next[(size_t)i] >= 0 && plain(gates[(size_t)next[(size_t)i]])) {
+                const cd a(g.a[0], g.a[1]), d(g.d[0], g.d[1]);
+                if (std::abs(std::abs(a) - 1.0) < 0.5 && std::abs(scale) >= least) {
+                    scale *= a;
+                    phase[q] *= d / a;
+                    continue;
+                }
+            }
+            out.push_back(g);
+            continue;
+        }
+        const cd a(g.a[0], g.a[1]), b = cd(g.b[0], g.b[1]) * phase[q], c(g.c[0], g.c[1]),
+                 d = cd(g.d[0], g.d[1]) * phase[q];
+        phase[q] = cd(1.0, 0.0);
+        qm_gate o = g;
+        o.kernel = QM_KERNEL_MATRIX;
+        const bool form_b = std::abs(a) < std::abs(c);
+        const cd big = form_b ? c : a, other = form_b ? a : c;
+        const double m = std::abs(big);
+        const long nx = next[(size_t)i];
+        bool split = nx >= 0 && plain(gates[(size_t)nx]) && i != last_plain && m > 0.0 && std::isfinite(m) &&
+                     std::abs(scale) * m >= least;
+        if (split) {
+            // column 0 = big (1, t phi) with the larger entry first; phi = 1 when t = 0
+            const double t = std::abs(other) / m;
+            const cd gph = big / m;
+            // form A: a = g m, c = g phi m t; form B: a = g m t, c = g phi m
+            cd phi(1.0, 0.0), g0 = gph;
+            if (!form_b) {
+                if (t > 0.0) phi = (other / std::abs(other)) / gph;
+            } else {
+                if (t > 0.0) g0 = other / std::abs(other);
+                phi = gph / g0;
+            }
+            // column 1 = g (-m t lambda, phi m lambda) in form A, g (-m lambda, phi m t lambda) in form B
+            const cd lambda = form_b ? -b / (g0 * m) : d / (g0 * phi * m);
+            const cd want_b = form_b ? -lambda : -t * lambda, want_d = form_b ? t * lambda : lambda;
+            const double err = std::max(std::abs(g0 * m * want_b - b), std::abs(g0 * phi * m * want_d - d));
+            split = std::isfinite(err) && err <= 1e-15 * m;
+            if (split) {
+                set(o.a, cd(form_b ? t : 1.0, 0.0));
+                set(o.c, cd(form_b ? 1.0 : t, 0.0));
+                set(o.b, want_b);
+                set(o.d, want_d);
+                phase[q] = phi;
+                scale *= g0 * m;
+            }
+        }
+        if (!split) {
+            set(o.a, a * scale);
+            set(o.b, b * scale);
+            set(o.c, c * scale);
+            set(o.d, d * scale);
+            scale = cd(1.0, 0.0);
+        }
+        out.push_back(o);
+    }
+    for (int q = 0; q < 32; ++q) flush(q);
+    return out;
+}
+
+std::vector<qm_gate> one_shot_gates(const std::vector<qm_gate>& gates, int precision) {
+    return real_columns(cz_rewrite_enabled() ? cnots_as_cz(gates) : gates, precision);
+}
+
 bool plan_fused(const std::vector<qm_gate>& in, int qubits, int precision, int width, Plan& plan,
-                std::string& error, const std::vector<int32_t>* slots) {
+                std::string& error, const std::vector<int32_t>* slots, bool relabel) {
     std::vector<qm_gate> rewritten;
     const bool rewrite = !slots && cz_rewrite_enabled() && (width == 0 || width >= 9);
     if (rewrite) rewritten = cnots_as_cz(in);
     const std::vector<qm_gate>& gates = rewrite ? rewritten : in;
     if (!plan_fused_with(gates, qubits, precision, width, plan, error, slots, false)) return false;
-    if (slots || !relabel_enabled() || plan.width == 1 || plan.passes.size() < 2) return true;
+    if (slots || !relabel || !relabel_enabled() || plan.width == 1 || plan.passes.size() < 2) return true;
     Plan alt;
     std::string alt_error;
     if (plan_fused_with(gates, qubits, precision, width, alt, alt_error, slots, true) &&
