@@ -1971,10 +1971,21 @@ cudaError_t launch_plan_pass(const Plan& plan, size_t pass, void* amps, const Fu
 }
 
 // ---------------------------------------------------------------- tiled expectation, compiled
-// The tiled expectation kernel (qm_expect.cu) generated for one tile pass's term list: flip
-// masks, pivots, phases and the tile-local Z-sign bits are constants, so a flip group's loop is
-// two shared loads, the FP64 overlap and one add or subtract per term.  The reduction order and
-// the partial-table layout are those of the generic kernel.
+// The tiled expectation kernel (qm_expect.cu) generated for one tile pass's term list, with the
+// generic kernel's partial-table layout.  Each of the 2^(k-4) threads holds 16 amplitudes:
+//   - diagonal terms: a Walsh-Hadamard transform of the tile's probabilities, four bits at a time
+//     in registers, exchanged through shared memory in between (fewer than three terms: summed);
+//   - flips of one to four tile bits: stages that put them on the register index, so a flip pairs
+//     registers of one thread and signs on register bits are the sign of an add.  A stage reads the
+//     tile once for all its terms (the first one, on the load layout, not at all);
+//   - wider flips and terms whose phase does not match their signs: pairs read from the tile.
+// A warp's sums are reduced up to eight at a time, half of them changing lanes at each step (18
+// shuffles for eight sums against 80).
+// Bound: shared-memory reads, shuffles and (complex64) the widening of each amplitude per stage,
+// about as much as the FP64 adds.  Pairs read from the tile for every flip, and a transform that
+// exchanged each bit, kept the shared-memory pipe 83 % busy: 32 complex64 states of 18 qubits, XXZ
+// chain of 69 terms, took 107 + 40 us for the two passes, and 52 + 24 us now.  Three blocks per SM for
+// complex64 (two: 57 + 30 us, 128 registers; 80 now); complex128 would spill at three.
 namespace {
 
 uint32_t insert_zero(uint32_t v, int bit) {
@@ -1991,171 +2002,309 @@ std::string generate_expect(int qubits, bool fp64, const TilePass& tp, const Til
     for (int b = 0; b < K - R; ++b) thread_mask |= 1u << tp.q[b];
     for (int m = 0; m < R; ++m) reg_g[m] = 1u << tp.q[K - R + m];
     const uint32_t all = qubits >= 32 ? 0xffffffffu : ((1u << qubits) - 1u);
-    const uint32_t outer_all = all & ~tp.block_mask;
+    const uint32_t outer_all = all & ~tp.block_mask, tile_all = (1u << K) - 1u;
     auto local_of = [&](uint32_t global) {
         uint32_t l = 0;
         for (int b = 0; b < K; ++b)
             if (global & (1u << tp.q[b])) l |= 1u << b;
         return l;
     };
-    const uint32_t lo_mask = (1u << (K - R)) - 1u;
+    auto sign_of = [&](int k) { return local_of(terms[k].sign & tp.block_mask); };
     int ndiag = 0;
     while (ndiag < T && terms[ndiag].flip_local == 0) ++ndiag;
     const bool wht = ndiag >= 3;
 
-    std::ostringstream os;
-    os << "typedef unsigned int u32;\ntypedef unsigned long long u64;\n";
-    os << "typedef " << (fp64 ? "double2" : "float2") << " V;\n";
-    os << "struct ExpLaunch { u32 outer_mask; int row_offset; int rows_per_state; int columns; int mass_column; int pad;\n"
-          "  u64 state_stride; double* partials; };\n";
-    os << "__device__ __forceinline__ u32 qm_deposit(u32 value, u32 mask) {\n"
-          "  u32 out = 0;\n"
-          "  while (mask) { const u32 low = mask & (0u - mask); if (value & 1u) out |= low; value >>= 1; mask ^= low; }\n"
-          "  return out;\n}\n";
-    os << "__device__ __forceinline__ double warp_sum(double v) {\n"
-          "  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);\n  return v;\n}\n";
-    // per-term constants of the final write
-    os << "__constant__ int c_col[" << std::max(1, T) << "] = {";
-    for (int k = 0; k < T; ++k) os << (k ? ", " : "") << terms[k].column;
-    os << "};\n__constant__ u32 c_loc[" << std::max(1, T) << "] = {";
-    for (int k = 0; k < T; ++k) os << (k ? ", " : "") << hexu(local_of(terms[k].sign & tp.block_mask));
-    os << "};\n__constant__ u32 c_sout[" << std::max(1, T) << "] = {";
-    for (int k = 0; k < T; ++k) os << (k ? ", " : "") << hexu(terms[k].sign & outer_all);
-    os << "};\n";
-    os << "extern \"C\" __global__ void __launch_bounds__(" << NT << ", " << std::max(1, 512 / NT)
-       << ") qm_expect(const V* __restrict__ s, const __grid_constant__ ExpLaunch P) {\n";
-    os << "extern __shared__ __align__(16) unsigned char smem_raw[];\n";
-    os << "V* tile = reinterpret_cast<V*>(smem_raw);\n";
-    os << "double* red = reinterpret_cast<double*>(smem_raw + " << ((fp64 ? 16 : 8) << K) << ");\n";
-    os << "const u32 t = threadIdx.x;\nconst int warp = t >> 5, lane = t & 31;\n(void)warp; (void)lane;\n";
-    os << "s += (u64)blockIdx.y * P.state_stride;\n";
+    // flip groups of at most eight terms, and the stage (four tile bits on the register index,
+    // ascending) that takes each; -1: pairs read from the tile
+    struct Group {
+        int first, count, stage;
+        bool paired;
+    };
+    std::vector<Group> groups;
+    for (int k = ndiag; k < T;) {
+        Group g{k, 0, -1, true};
+        const uint32_t F = terms[k].flip_local;
+        for (; g.count < 8 && k < T && terms[k].flip_local == F; ++g.count, ++k)
+            if (((__builtin_popcount(F & sign_of(k)) ^ terms[k].phase) & 1) != 0) g.paired = false;
+        groups.push_back(g);
+    }
+    const uint32_t load_layout = tile_all & ~((1u << (K - R)) - 1u);
+    std::vector<uint32_t> stages;
+    for (size_t a = 0; a < groups.size(); ++a) {
+        if (groups[a].stage >= 0) continue;
+        uint32_t layout = 0;
+        for (size_t b = a; b < groups.size(); ++b) {
+            const uint32_t l = layout | terms[groups[b].first].flip_local;
+            if (groups[b].stage >= 0 || !groups[b].paired || __builtin_popcount(l) > R) continue;
+            layout = l;
+            groups[b].stage = (int)stages.size();
+        }
+        if (!layout) continue;
+        for (int b = K - 1; __builtin_popcount(layout) < R; --b) layout |= 1u << b;
+        stages.push_back(layout);
+    }
+
+    std::ostringstream os;  // the kernel's body
+    std::vector<int> column;  // of each sum in a warp's row
+    std::vector<std::pair<std::string, int>> sums;  // waiting to be reduced: value, column (-1: the mass)
+    auto parity = [&](const std::string& index, uint32_t bits, uint32_t outer_bits) {
+        std::string e;
+        if (bits) e = "__popc(" + index + " & " + hexu(bits) + ")";
+        if (outer_bits) e += std::string(e.empty() ? "" : " + ") + "__popc(outer & " + hexu(outer_bits) + ")";
+        return e;
+    };
+    auto reduce = [&]() {
+        const int n = (int)sums.size();
+        if (n == 0) return;
+        int H = 1;
+        while (H < n) H *= 2;
+        os << "{\n";
+        for (int i = 0; i < H; ++i) os << "double v" << i << " = " << (i < n ? sums[(size_t)i].first : "0.0") << ";\n";
+        int d = 16;
+        for (int h = H / 2; h >= 1; h /= 2, d /= 2) {
+            os << "{ const bool up = (lane & " << d << ") != 0;\n";
+            for (int i = 0; i < h; ++i)
+                os << "{ const double mine = up ? v" << i + h << " : v" << i << ", other = up ? v" << i << " : v" << i + h << "; v" << i
+                   << " = mine + __shfl_xor_sync(0xffffffffu, other, " << d << "); }\n";
+            os << "}\n";
+        }
+        for (; d >= 1; d /= 2) os << "v0 += __shfl_xor_sync(0xffffffffu, v0, " << d << ");\n";
+        os << "if ((lane & " << 32 / H - 1 << ") == 0 && lane < " << n * (32 / H) << ") red[warp * " << NCOL << " + " << column.size()
+           << " + lane / " << 32 / H << "] = v0;\n}\n";
+        for (const auto& v : sums) column.push_back(v.second);
+        sums.clear();
+    };
+    auto take = [&](const std::string& value, const std::string& par, int col) {
+        sums.push_back({par.empty() ? value : "((" + par + ") & 1) ? -" + value + " : " + value, col});
+        if (sums.size() == 8) reduce();
+    };
+    auto X = [](int i) { return "x" + std::to_string(i); };
+    // names of the values that wait for a reduction stay in scope until the end of their stage
+    int uid = 0;
+
+    // the tile, 16 amplitudes per thread: threads on the low K - 4 bits
     os << "const u32 outer = qm_deposit(blockIdx.x, P.outer_mask);\n";
-    os << "{ const u32 g0 = outer | " << deposit_expr("t", thread_mask) << ";\n";
+    os << "const u64 row = (u64)blockIdx.y * P.rows_per_state + P.row_offset + blockIdx.x;\n";
+    os << "V ";
+    for (int i = 0; i < NR; ++i) os << (i ? ", " : "") << X(i);
+    os << ";\n{ const u32 g0 = outer | " << deposit_expr("t", thread_mask) << ";\n";
     for (int i = 0; i < NR; ++i) {
         uint32_t off = 0;
         for (int m = 0; m < R; ++m)
             if ((i >> m) & 1) off |= reg_g[m];
-        os << "tile[t | " << hexu((uint32_t)i << (K - R)) << "] = s[g0 | " << hexu(off) << "];\n";
+        os << X(i) << " = s[g0 | " << hexu(off) << "];\n";
     }
-    os << "}\n__syncthreads();\n";
-
-    // flip groups (and diagonal terms when fewer than three), at most 8 terms per loop
-    for (int k = wht ? ndiag : 0; k < T;) {
-        const uint32_t F = terms[k].flip_local;
-        int cnt = 1;
-        while (cnt < 8 && k + cnt < T && terms[k + cnt].flip_local == F) ++cnt;
-        bool paired = F != 0;
-        for (int u = 0; u < cnt; ++u) {
-            const uint32_t sl = local_of(terms[k + u].sign & tp.block_mask);
-            if (((__builtin_popcount(F & sl) ^ terms[k + u].phase) & 1) != 0) paired = false;
-        }
-        os << "{\n";
-        for (int u = 0; u < cnt; ++u) os << "double a" << u << " = 0.0;\n";
-        auto term_add = [&](int u, uint32_t j_const, const char* ore, const char* oim) {
-            const TileTerm& tt = terms[k + u];
-            const uint32_t sl = local_of(tt.sign & tp.block_mask);
-            const bool neg = (tt.phase == 1 || tt.phase == 2) ^ (__builtin_popcount(j_const & sl) & 1);
-            os << "a" << u << (neg ? " -= " : " += ") << ((tt.phase & 1) ? oim : ore) << ";\n";
+    os << "}\n";
+    if (ndiag > 0 || tp.with_mass) {
+        os << "{\ndouble w[" << NR << "];\n";
+        for (int i = 0; i < NR; ++i)
+            os << "w[" << i << "] = (double)" << X(i) << ".x * " << X(i) << ".x + (double)" << X(i) << ".y * " << X(i) << ".y;\n";
+        auto total = [&](const std::string& name, uint32_t sign, bool negate) {
+            os << "double " << name << " = " << (negate ? "-" : "") << "w[0];\n";
+            for (int i = 1; i < NR; ++i)
+                os << name << (negate ^ (__builtin_popcount(((uint32_t)i << (K - R)) & sign) & 1) ? " -= w[" : " += w[") << i << "];\n";
         };
-        std::string jt;
-        uint32_t jt_bits = lo_mask;  // local bits the run-time index part can hold
-        if (paired) {
-            const int pivot = 31 - __builtin_clz(F);
-            if (pivot >= K - R) {
-                jt = "t";
-            } else {
-                jt_bits = (lo_mask << 1) | 1u;  // the thread index with a zero inserted at the pivot
-                const uint32_t below = (1u << pivot) - 1u;
-                os << "const u32 jt = (t & " << hexu(below) << ") | ((t & " << hexu(~below & lo_mask) << ") << 1);\n";
-                jt = "jt";
-            }
-            for (int r = 0; r < NR / 2; ++r) {
-                const uint32_t c = insert_zero((uint32_t)(NT * r), pivot);
-                os << "{ const V a = tile[" << jt << " | " << hexu(c) << "], b = tile[(" << jt << " | " << hexu(c) << ") ^ "
-                   << hexu(F) << "];\n";
-                os << "const double ar = a.x, ai = a.y, br = b.x, bi = b.y;\n";
-                os << "const double ore = br * ar + bi * ai, oim = br * ai - bi * ar;\n";
-                for (int u = 0; u < cnt; ++u) term_add(u, c, "ore", "oim");
-                os << "}\n";
-            }
-        } else {
-            jt = "t";
-            for (int i = 0; i < NR; ++i) {
-                const uint32_t c = (uint32_t)i << (K - R);
-                os << "{ const V a = tile[t | " << hexu(c) << "];\nconst double ar = a.x, ai = a.y;\n";
-                if (F == 0) {
-                    os << "const double ore = ar * ar + ai * ai, oim = 0.0;\n";
-                } else {
-                    os << "const V b = tile[(t | " << hexu(c) << ") ^ " << hexu(F) << "];\nconst double br = b.x, bi = b.y;\n";
-                    os << "const double ore = br * ar + bi * ai, oim = br * ai - bi * ar;\n";
+        if (tp.with_mass) {
+            total("mass", 0, false);
+            take("mass", "", -1);
+        }
+        for (int k = 0; !wht && k < ndiag; ++k) {
+            const std::string n = "d" + std::to_string(k);
+            const int phase = terms[k].phase;
+            if (phase & 1) os << "const double " << n << " = 0.0;\n";
+            else total(n, sign_of(k), phase == 2);
+            take(n, parity("t", sign_of(k) & (NT - 1u), terms[k].sign & outer_all), terms[k].column);
+        }
+        reduce();
+        if (wht) {
+            // the transform: register bits, exchange, the next four bits below, ...
+            os << "double* wbuf = reinterpret_cast<double*>(smem_raw);\n";
+            uint32_t done = 0, layout = load_layout;
+            std::string at = "t";
+            for (;;) {
+                int bit[R], n = 0;
+                for (int b = 0; b < K; ++b)
+                    if ((layout >> b) & 1u) bit[n++] = b;
+                auto index = [&](int i) {
+                    uint32_t c = 0;
+                    for (int m = 0; m < R; ++m)
+                        if ((i >> m) & 1) c |= 1u << bit[m];
+                    return hexu(swz_host(c, false));
+                };
+                os << "{ const u32 at = qm_swz8(" << at << ");\n";
+                if (done)
+                    for (int i = 0; i < NR; ++i) os << "w[" << i << "] = wbuf[at ^ " << index(i) << "];\n";
+                for (int m = 0; m < R; ++m) {
+                    if ((done >> bit[m]) & 1u) continue;
+                    for (int i = 0; i < NR; ++i)
+                        if (!((i >> m) & 1))
+                            os << "{ const double a = w[" << i << "], b = w[" << (i | (1 << m)) << "]; w[" << i << "] = a + b; w["
+                               << (i | (1 << m)) << "] = a - b; }\n";
                 }
-                for (int u = 0; u < cnt; ++u) term_add(u, c, "ore", "oim");
-                os << "}\n";
+                for (int i = 0; i < NR; ++i) os << "wbuf[at ^ " << index(i) << "] = w[" << i << "];\n";
+                os << "}\n__syncthreads();\n";
+                done |= layout;
+                if (done == tile_all) break;
+                const int next = std::max(0, K - R - __builtin_popcount(done));
+                layout = ((1u << R) - 1u) << next;
+                at = deposit_expr("t", tile_all & ~layout);
             }
-        }
-        for (int u = 0; u < cnt; ++u) {
-            const TileTerm& tt = terms[k + u];
-            const uint32_t sl = local_of(tt.sign & tp.block_mask) & jt_bits;  // run-time part of the local sign
-            const uint32_t so = tt.sign & outer_all;
-            std::string par;
-            if (sl) par = "__popc(" + jt + " & " + hexu(sl) + ")";
-            if (so) par += std::string(par.empty() ? "" : " + ") + "__popc(outer & " + hexu(so) + ")";
-            const char* scale = paired ? "2.0" : "1.0";
-            if (par.empty())
-                os << "{ const double v = warp_sum(" << scale << " * a" << u << ");\n";
-            else
-                os << "{ const double v = warp_sum(((" << par << ") & 1) ? -" << scale << " * a" << u << " : " << scale
-                   << " * a" << u << ");\n";
-            os << "if (lane == 0) red[warp * " << NCOL << " + " << (k + u) << "] = v; }\n";
-        }
-        os << "}\n";
-        k += cnt;
-    }
-    if (tp.with_mass) {
-        os << "{ double m = 0.0;\n";
-        for (int i = 0; i < NR; ++i)
-            os << "{ const V a = tile[t | " << hexu((uint32_t)i << (K - R)) << "]; m += (double)a.x * a.x + (double)a.y * a.y; }\n";
-        os << "m = warp_sum(m);\nif (lane == 0) red[warp * " << NCOL << " + " << T << "] = m; }\n";
-    }
-    if (wht) {
-        // Walsh-Hadamard transform of the tile's Born probabilities (as the generic kernel)
-        os << "double* wbuf = reinterpret_cast<double*>(smem_raw);\n{\ndouble w[" << NR << "];\n";
-        for (int i = 0; i < NR; ++i)
-            os << "{ const V a = tile[t | " << hexu((uint32_t)i << (K - R)) << "]; w[" << i
-               << "] = (double)a.x * a.x + (double)a.y * a.y; }\n";
-        for (int m = 0; m < R; ++m)
-            for (int i = 0; i < NR; ++i)
-                if (!((i >> m) & 1))
-                    os << "{ const double x = w[" << i << "], y = w[" << (i | (1 << m)) << "]; w[" << i << "] = x + y; w["
-                       << (i | (1 << m)) << "] = x - y; }\n";
-        for (int m = 0; m < 5; ++m) {
-            os << "#pragma unroll\nfor (int i = 0; i < " << NR << "; ++i) { const double y = __shfl_xor_sync(0xffffffffu, w[i], "
-               << (1 << m) << "); w[i] = ((lane >> " << m << ") & 1) ? y - w[i] : w[i] + y; }\n";
-        }
-        os << "__syncthreads();\n";
-        os << "#pragma unroll\nfor (int i = 0; i < " << NR << "; ++i) wbuf[t | ((u32)i << " << (K - R) << ")] = w[i];\n";
-        for (int m = 5; m < K - R; ++m) {
-            os << "__syncthreads();\n#pragma unroll\nfor (int i = 0; i < " << NR << "; ++i) { const u32 j = t | ((u32)i << "
-               << (K - R) << "); const double x = wbuf[j], y = wbuf[j ^ " << (1u << m) << "u]; w[i] = ((j >> " << m
-               << ") & 1u) ? y - x : x + y; }\n";
-            os << "__syncthreads();\n#pragma unroll\nfor (int i = 0; i < " << NR << "; ++i) wbuf[t | ((u32)i << " << (K - R)
-               << ")] = w[i];\n";
+            os << "if (t < " << ndiag << ") for (int k = t; k < " << ndiag << "; k += " << NT << ") {\n"
+                  "double sum = wbuf[c_loc[k]];\nif (__popc(outer & c_sout[k]) & 1) sum = -sum;\n"
+                  "P.partials[row * P.columns + c_diag[k]] = sum;\n}\n";
+            if (!groups.empty()) os << "__syncthreads();\n";
         }
         os << "}\n";
     }
-    os << "__syncthreads();\n";
-    os << "const u64 row = (u64)blockIdx.y * P.rows_per_state + P.row_offset + blockIdx.x;\n";
-    os << "for (int k = t; k < " << (T + (tp.with_mass ? 1 : 0)) << "; k += " << NT << ") {\n";
-    os << "double sum = 0.0;\n";
-    if (wht) {
-        os << "if (k < " << ndiag << ") { sum = reinterpret_cast<const double*>(smem_raw)[c_loc[k]];\n"
-              "  if (__popc(outer & c_sout[k]) & 1) sum = -sum;\n"
-              "  P.partials[row * P.columns + c_col[k]] = sum; continue; }\n";
+    if (!groups.empty()) {
+        os << "V* tile = reinterpret_cast<V*>(smem_raw);\n{ const u32 at = qm_swz(t);\n";
+        for (int i = 0; i < NR; ++i)
+            os << "tile[at ^ " << hexu(swz_host((uint32_t)i << (K - R), fp64)) << "] = " << X(i) << ";\n";
+        os << "}\n";
     }
-    os << "for (int w = 0; w < " << WARPS << "; ++w) sum += red[w * " << NCOL << " + k];\n";
-    os << "const int col = k < " << T << " ? c_col[k < " << T << " ? k : 0] : P.mass_column;\n";
-    os << "P.partials[row * P.columns + col] = sum;\n}\n}\n";
-    return os.str();
+    auto add = [&](const std::string& name, const TileTerm& tt, uint32_t at, uint32_t sl, bool first, const char* ore,
+                   const char* oim) {
+        const bool neg = (tt.phase == 1 || tt.phase == 2) ^ (__builtin_popcount(at & sl) & 1);
+        const char* v = (tt.phase & 1) ? oim : ore;
+        if (first) os << name << " = " << (neg ? "-" : "") << v << ";\n";
+        else os << name << (neg ? " -= " : " += ") << v << ";\n";
+    };
+    // the stage on the load layout first: its amplitudes are in registers
+    std::vector<int> order(stages.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return (stages[x] == load_layout) > (stages[y] == load_layout); });
+    bool synced = false;
+    for (int st : order) {
+        const uint32_t layout = stages[(size_t)st], lanes = tile_all & ~layout;
+        int bit[R], n = 0;
+        for (int b = 0; b < K; ++b)
+            if ((layout >> b) & 1u) bit[n++] = b;
+        auto at_of = [&](int i) {
+            uint32_t c = 0;
+            for (int m = 0; m < R; ++m)
+                if ((i >> m) & 1) c |= 1u << bit[m];
+            return c;
+        };
+        if (layout != load_layout) {
+            if (!synced) os << "__syncthreads();\n";
+            synced = true;
+        }
+        os << "{ const u32 base = " << deposit_expr("t", lanes) << ";\n";
+        if (layout != load_layout) {
+            os << "const u32 at = qm_swz(base);\n";
+            for (int i = 0; i < NR; ++i) os << X(i) << " = tile[at ^ " << hexu(swz_host(at_of(i), fp64)) << "];\n";
+        }
+        for (int i = 0; i < NR; ++i)
+            os << "const double r" << i << " = " << X(i) << ".x, i" << i << " = " << X(i) << ".y;\n";
+        for (const Group& g : groups) {
+            if (g.stage != st) continue;
+            if (sums.size() + g.count > 8) reduce();
+            const uint32_t F = terms[g.first].flip_local;
+            int flip = 0;
+            for (int m = 0; m < R; ++m)
+                if ((F >> bit[m]) & 1u) flip |= 1 << m;
+            const int pivot = 31 - __builtin_clz((unsigned)flip), id = uid;
+            uid += g.count;
+            os << "double ";
+            for (int u = 0; u < g.count; ++u) os << (u ? ", " : "") << "a" << id + u;
+            os << ";\n";
+            bool re = false, im = false;
+            for (int u = 0; u < g.count; ++u) ((terms[g.first + u].phase & 1) ? im : re) = true;
+            bool first = true;
+            for (int i = 0; i < NR; ++i) {
+                if ((i >> pivot) & 1) continue;
+                const int k = i ^ flip;
+                os << "{ ";
+                if (re) os << "const double ore = r" << k << " * r" << i << " + i" << k << " * i" << i << ";\n";
+                if (im) os << "const double oim = r" << k << " * i" << i << " - i" << k << " * r" << i << ";\n";
+                for (int u = 0; u < g.count; ++u)
+                    add("a" + std::to_string(id + u), terms[g.first + u], at_of(i), sign_of(g.first + u), first, "ore", "oim");
+                os << "}\n";
+                first = false;
+            }
+            for (int u = 0; u < g.count; ++u)  // a pair's two members contribute the same
+                take("2.0 * a" + std::to_string(id + u),
+                     parity("base", sign_of(g.first + u) & lanes, terms[g.first + u].sign & outer_all), terms[g.first + u].column);
+        }
+        reduce();
+        os << "}\n";
+    }
+    for (const Group& g : groups) {
+        if (g.stage >= 0) continue;
+        if (!synced) os << "__syncthreads();\n";
+        synced = true;
+        const uint32_t F = terms[g.first].flip_local;
+        // a pair is visited once where both members contribute the same
+        const int pivot = g.paired ? 31 - __builtin_clz(F) : -1;
+        const uint32_t lo = NT - 1u;
+        os << "{ const u32 jt = ";
+        uint32_t jt_bits = lo;
+        if (!g.paired || pivot >= K - R) {
+            os << "t";
+        } else {
+            const uint32_t below = (1u << pivot) - 1u;
+            jt_bits = (lo << 1) | 1u;
+            os << "(t & " << hexu(below) << ") | ((t & " << hexu(~below & lo) << ") << 1)";
+        }
+        os << ", at = qm_swz(jt);\n";
+        for (int u = 0; u < g.count; ++u) os << "double a" << u << " = 0.0;\n";
+        for (int r = 0; r < (g.paired ? NR / 2 : NR); ++r) {
+            const uint32_t c = g.paired ? insert_zero((uint32_t)(NT * r), pivot) : (uint32_t)(NT * r);
+            os << "{ const V a = tile[at ^ " << hexu(swz_host(c, fp64)) << "], b = tile[at ^ " << hexu(swz_host(c ^ F, fp64)) << "];\n";
+            os << "const double ar = a.x, ai = a.y, br = b.x, bi = b.y;\n";
+            os << "const double ore = br * ar + bi * ai, oim = br * ai - bi * ar;\n(void)ore; (void)oim;\n";
+            for (int u = 0; u < g.count; ++u)
+                add("a" + std::to_string(u), terms[g.first + u], c, sign_of(g.first + u), false, "ore", "oim");
+            os << "}\n";
+        }
+        for (int u = 0; u < g.count; ++u)
+            take((g.paired ? "2.0 * a" : "a") + std::to_string(u),
+                 parity("jt", sign_of(g.first + u) & jt_bits, terms[g.first + u].sign & outer_all), terms[g.first + u].column);
+        reduce();
+        os << "}\n";
+    }
+    if (!column.empty()) {
+        os << "__syncthreads();\nfor (int k = t; k < " << column.size() << "; k += " << NT << ") {\ndouble sum = 0.0;\n";
+        os << "for (int w = 0; w < " << WARPS << "; ++w) sum += red[w * " << NCOL << " + k];\n";
+        os << "const int col = c_col[k];\nP.partials[row * P.columns + (col < 0 ? P.mass_column : col)] = sum;\n}\n";
+    }
+
+    std::ostringstream hd;
+    hd << "typedef unsigned int u32;\ntypedef unsigned long long u64;\n";
+    hd << "typedef " << (fp64 ? "double2" : "float2") << " V;\n";
+    hd << "struct ExpLaunch { u32 outer_mask; int row_offset; int rows_per_state; int columns; int mass_column; int pad;\n"
+          "  u64 state_stride; double* partials; };\n";
+    hd << "__device__ __forceinline__ u32 qm_deposit(u32 value, u32 mask) {\n"
+          "  u32 out = 0;\n"
+          "  while (mask) { const u32 low = mask & (0u - mask); if (value & 1u) out |= low; value >>= 1; mask ^= low; }\n"
+          "  return out;\n}\n";
+    // the slot swizzles of 16-byte and 8-byte values
+    hd << "__device__ __forceinline__ u32 qm_swz8(u32 j) { const u32 h = j >> 4; return j ^ ((h ^ (h >> 4) ^ (h >> 8)) & 15u); }\n";
+    if (fp64)
+        hd << "__device__ __forceinline__ u32 qm_swz(u32 j) { const u32 h = j >> 3; return j ^ ((h ^ (h >> 3) ^ (h >> 6) ^ (h >> 9)) "
+              "& 7u); }\n";
+    else
+        hd << "#define qm_swz qm_swz8\n";
+    auto table = [&](const char* type, const char* name, size_t n, auto value) {
+        hd << "__constant__ " << type << " " << name << "[" << std::max<size_t>(1, n) << "] = {";
+        for (size_t k = 0; k < n; ++k) hd << (k ? ", " : "") << value((int)k);
+        hd << "};\n";
+    };
+    // of each reduced sum: its column; of each transformed term: its column, its place, its outer signs
+    table("int", "c_col", column.size(), [&](int k) { return column[(size_t)k]; });
+    if (wht) {
+        table("int", "c_diag", (size_t)ndiag, [&](int k) { return terms[k].column; });
+        table("u32", "c_loc", (size_t)ndiag, [&](int k) { return hexu(swz_host(sign_of(k), false)); });
+        table("u32", "c_sout", (size_t)ndiag, [&](int k) { return hexu(terms[k].sign & outer_all); });
+    }
+    hd << "extern \"C\" __global__ void __launch_bounds__(" << NT << ", " << (fp64 ? 512 : 768) / NT
+       << ") qm_expect(const V* __restrict__ s, const __grid_constant__ ExpLaunch P) {\n";
+    hd << "extern __shared__ __align__(16) unsigned char smem_raw[];\n";
+    hd << "double* red = reinterpret_cast<double*>(smem_raw + " << ((fp64 ? 16 : 8) << K) << ");\n";
+    hd << "const u32 t = threadIdx.x;\nconst int warp = t >> 5, lane = t & 31;\n(void)warp; (void)lane; (void)red;\n";
+    hd << "s += (u64)blockIdx.y * P.state_stride;\n";
+    return hd.str() + os.str() + "}\n";
 }
 
 struct ExpLaunchHost {
