@@ -283,6 +283,7 @@ __device__ __forceinline__ u32 qm_deposit(u32 value, u32 mask) {
 // (dr, di) = a * (br, bi) + (cr, ci) and a * (br, bi): one issue slot for two multiply-adds, at the
 // rate of two (complex64 passes wait for issue slots before they wait for the FP32 pipe: 71 % against
 // 58 % busy in a 27-qubit brick pass).  A plan of 27 qubits and depth 17 went from 13.03 to 12.03 ms.
+// A rotation's pair (x, y) from x and w: a: (x + n w, t x + w); b: (t x + w, x + n w).
 #ifdef QM_EMULATED
 inline void qm_fma2(float& dr, float& di, float a, float br, float bi, float cr, float ci) {
     dr = a * br + cr;
@@ -291,6 +292,16 @@ inline void qm_fma2(float& dr, float& di, float a, float br, float bi, float cr,
 inline void qm_mul2(float& dr, float& di, float a, float br, float bi) {
     dr = a * br;
     di = a * bi;
+}
+inline void qm_rotate_a(float& xr, float& xi, float& yr, float& yi, float t, float n, float wr, float wi) {
+    const float r = xr, i = xi;
+    qm_fma2(xr, xi, n, wr, wi, r, i);
+    qm_fma2(yr, yi, t, r, i, wr, wi);
+}
+inline void qm_rotate_b(float& xr, float& xi, float& yr, float& yi, float t, float n, float wr, float wi) {
+    const float r = xr, i = xi;
+    qm_fma2(xr, xi, t, r, i, wr, wi);
+    qm_fma2(yr, yi, n, wr, wi, r, i);
 }
 #else
 // macros: NVRTC takes a third longer over the same as functions
@@ -301,6 +312,14 @@ inline void qm_mul2(float& dr, float& di, float a, float br, float bi) {
 #define qm_mul2(dr, di, a, br, bi)                                                                            \
     asm("{ .reg .b64 a, b; mov.b64 a, {%2, %2}; mov.b64 b, {%3, %4}; mul.rn.f32x2 b, a, b; mov.b64 {%0, %1}, b; }" \
         : "=f"(dr), "=f"(di) : "f"(a), "f"(br), "f"(bi))
+#define qm_rotate(first, second, xr, xi, yr, yi, t, n, wr, wi)                                                \
+    asm("{ .reg .b64 t, n, x, w, u; mov.b64 t, {%4, %4}; mov.b64 n, {%5, %5}; mov.b64 w, {%6, %7};\n"         \
+        "mov.b64 x, {%0, %1};\n" first second "}"                                                             \
+        : "+f"(xr), "+f"(xi), "=f"(yr), "=f"(yi) : "f"(t), "f"(n), "f"(wr), "f"(wi))
+#define qm_rotate_a(...)                                                                                      \
+    qm_rotate("fma.rn.f32x2 u, n, w, x; mov.b64 {%0, %1}, u;\n", "fma.rn.f32x2 u, t, x, w; mov.b64 {%2, %3}, u;\n", __VA_ARGS__)
+#define qm_rotate_b(...)                                                                                      \
+    qm_rotate("fma.rn.f32x2 u, t, x, w; mov.b64 {%0, %1}, u;\n", "fma.rn.f32x2 u, n, w, x; mov.b64 {%2, %3}, u;\n", __VA_ARGS__)
 #endif
 #ifndef QM_EMULATED
 // tile copies (cp.async, no registers) and the named barriers of two-team blocks
@@ -993,8 +1012,12 @@ struct Gen {
         for (int i = 0; i < NR; ++i) {
             if ((i >> M) & 1) continue;
             const int k = i | (1 << M);
-            os << "{ const " << T << " xr = " << X(i) << ", xi = " << Y(i) << ";\n";
-            if (P.cls == 0)
+            os << "{ ";
+            if (!packed) os << "const " << T << " xr = " << X(i) << ", xi = " << Y(i) << ";\n";
+            std::string w = "wr, wi";
+            if (P.cls == 0 && packed)
+                w = X(k) + ", " + Y(k);
+            else if (P.cls == 0)
                 os << "const " << T << " wr = " << X(k) << ", wi = " << Y(k) << ";\n";
             else if (P.cls == 1 && packed)
                 os << "float wr, wi; qm_mul2(wr, wi, -1.0f, " << X(k) << ", " << Y(k) << ");\n";
@@ -1017,11 +1040,8 @@ struct Gen {
                    << "), wi = " << s << "(" << P.re[i] << " * " << Y(k) << " + " << P.im[i] << " * " << X(k) << ");\n";
             }
             if (packed) {
-                const std::string xi = X(i) + ", " + Y(i) + ", ", xk = X(k) + ", " + Y(k) + ", ";
-                if (!sp.form_b)
-                    os << "qm_fma2(" << xi << "n, wr, wi, xr, xi); qm_fma2(" << xk << "t, xr, xi, wr, wi); }\n";
-                else
-                    os << "qm_fma2(" << xi << "t, xr, xi, wr, wi); qm_fma2(" << xk << "n, wr, wi, xr, xi); }\n";
+                os << (sp.form_b ? "qm_rotate_b(" : "qm_rotate_a(") << X(i) << ", " << Y(i) << ", " << X(k) << ", " << Y(k)
+                   << ", t, n, " << w << "); }\n";
             } else if (!sp.form_b)
                 os << X(i) << " = xr - t * wr; " << Y(i) << " = xi - t * wi; " << X(k) << " = t * xr + wr; " << Y(k)
                    << " = t * xi + wi; }\n";
