@@ -533,6 +533,7 @@ struct VqeProblem {
         if (!plan_fused(gates, exec_qubits, precision, ctx->fusion_width, plan, err, &slots))
             return fail(QM_E_ARG, "planner: " + err);
         plan.start_zero = true;  // every circuit starts from |0...0>
+        plan.table_rotations = true;  // RY by a parameter, or by it and a shift
         jit_prepare(plan);       // one structure for every circuit of every wave
         if (!plan.ops.empty()) {
             program_bytes = plan.ops.size() * sizeof(FusedOp);

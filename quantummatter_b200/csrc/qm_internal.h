@@ -164,6 +164,8 @@ struct Plan {
     // so the caller's reset can be skipped.
     bool start_zero = false;
     bool zero_fused = false;
+    // Every real matrix that takes its coefficients from the batch table is a rotation [c -s; s c].
+    bool table_rotations = false;
     bool borrowed = false;          // d_ops belongs to a context buffer
     bool small = false;             // the gates run in one block, kSmallGates a launch (launch_small)
     std::vector<DenseOp> dense;         // dense fused gates (widths 2..6)

@@ -569,6 +569,79 @@ struct Gen {
         return {"fr" + n, "fi" + n, false};
     }
 
+    // What a block forms when it turns to another state, next to the state's coefficient rows:
+    //   - rotations whose angle comes from the table (real, uncontrolled; the plan says that they are
+    //     rotations): (s / c, 1) or (c / s, 0) in place of the row, whichever is at most 1, which is half
+    //     the multiply-adds of a 2x2 product.  The factors c or s left out are at least 0.7 each; their
+    //     product goes into the pass's last such matrix, which stays a 2x2 product.
+    //   - complex64: a diagonal group's 16 register phases, when all its members on register bits come
+    //     from the table: the same for every thread and tile.  They lie in the second half of the space
+    //     of the rows, which the launch sizes for doubles.
+    // 32 states of 18 qubits, 4 layers of RY, RZ and CZ: the passes took 237 us, and 201 us now (three
+    // shears a rotation instead: the same time, a third more rounding error).
+    std::vector<uint32_t> rotation_slots;
+    int scaled_slot = -1;
+    size_t phase_room = 0;  // groups that fit
+    std::vector<std::vector<uint32_t>> phase_groups;  // members: 4 * slot + register bit
+    bool table_rotation(const FusedOp& op) const {
+        return scaled_slot >= 0 && op.code == OP_MATRIX_REAL && (op.flags & kOpTable) &&
+               std::find(rotation_slots.begin(), rotation_slots.end(), op.reserved) != rotation_slots.end();
+    }
+    void rotate_by_table(const FusedOp& op) {
+        const std::string at = std::to_string(8 * op.reserved);
+        os << "{ const " << T << " t = table[" << at << "];\nif (table[" << at << " + 1] != (" << T << ")0) {\n";
+        for (int form = 0; form < 2; ++form) {
+            if (form == 0) os << "const " << T << " n = -t;\n";
+            for (int i = 0; i < NR; ++i) {
+                if ((i >> op.reg) & 1) continue;
+                const std::string xr = X(i), xi = Y(i), yr = X(i | (1 << op.reg)), yi = Y(i | (1 << op.reg));
+                if (form == 0 && !fp64)
+                    os << "qm_rotate_a(" << xr << ", " << xi << ", " << yr << ", " << yi << ", t, n, " << yr << ", " << yi << ");\n";
+                else if (form == 0)
+                    os << "{ const double r = " << xr << ", i = " << xi << "; " << xr << " = r + n * " << yr << "; " << xi
+                       << " = i + n * " << yi << "; " << yr << " = t * r + " << yr << "; " << yi << " = t * i + " << yi << "; }\n";
+                else
+                    os << "{ const " << T << " r = " << xr << ", i = " << xi << "; " << xr << " = t * r - " << yr << "; " << xi
+                       << " = t * i - " << yi << "; " << yr << " = t * " << yr << " + r; " << yi << " = t * " << yi << " + i; }\n";
+            }
+            os << (form == 0 ? "} else {\n" : "}\n}\n");
+        }
+    }
+    // the code that prepares them, and the lists it reads
+    std::string state_tables(int nt, std::ostringstream& lists) const {
+        std::ostringstream c;
+        if (scaled_slot >= 0) {
+            lists << "__constant__ u32 c_rotation[] = {";
+            for (uint32_t sl : rotation_slots) lists << sl << ", ";
+            lists << "};\n";
+            c << "if (t < 32u) { double g = 1.0;\nfor (u32 i = t; i < " << rotation_slots.size()
+              << "u; i += 32u) { const u32 at = 8u * c_rotation[i];\n"
+                 "const double c = __ldg(row + at), sn = __ldg(row + at + 4); const bool a = fabs(c) >= fabs(sn);\n"
+                 "table[at] = (" << T << ")(a ? sn / c : c / sn); table[at + 1] = (" << T << ")(a ? 1 : 0); g *= a ? c : sn; }\n"
+                 "for (int d = 16; d > 0; d >>= 1) g *= __shfl_xor_sync(0xffffffffu, g, d);\n"
+                 "if (t < 4u) table[" << 8 * scaled_slot << " + 2 * t] = (" << T << ")(g * __ldg(row + " << 8 * scaled_slot
+              << " + 2 * t)); }\n";
+        }
+        if (!phase_groups.empty()) {
+            std::ostringstream at;
+            size_t n = 0;
+            lists << "__constant__ u32 c_phase[] = {";
+            for (const auto& g : phase_groups) {
+                at << n << ", ";
+                for (uint32_t m : g) lists << m << ", ";
+                n += g.size();
+            }
+            lists << "};\n__constant__ u32 c_phase_at[] = {" << at.str() << n << "};\n";
+            c << "for (u32 i = t; i < " << NR * phase_groups.size() << "u; i += " << nt << ") { double re = 1.0, im = 0.0;\n"
+                 "for (u32 k = c_phase_at[i >> 4]; k < c_phase_at[(i >> 4) + 1]; ++k) { const u32 m = c_phase[k];\n"
+                 "const double* f = row + 8u * (m >> 2) + (((i >> (m & 3u)) & 1u) ? 6 : 0);\n"
+                 "const double fr = __ldg(f), fi = __ldg(f + 1), nr = re * fr - im * fi; im = re * fi + im * fr; re = nr; }\n"
+                 "V v; v.x = (" << T << ")re; v.y = (" << T << ")im; phases[i] = v; }\n";
+        }
+        if (!c.str().empty()) c << "__syncthreads();\n";
+        return c.str();
+    }
+
     // Commuting diagonals as one phase per register.  Members on thread or outer bits fold into one
     // factor u of the thread; members on register bits become a pair of factors per bit, and the
     // phases are products of two small tables (four members: 42 complex products against 80 with one
@@ -613,6 +686,15 @@ struct Gen {
             else
                 os << T << " ur = hr" << h << ", ui = hi" << h << ";\n";
         }
+        std::vector<uint32_t> members;
+        bool staged = phase_groups.size() < phase_room;
+        for (int k = 0; k < count; ++k) {
+            const FusedOp& m = ops[(size_t)(first + k)];
+            const int M = m.code == OP_DIAG && m.local >= 0 ? reg_of_local(m.local) : -1;
+            if (M >= 0 && !(m.flags & kOpTable)) staged = false;
+            if (M >= 0) members.push_back(4 * m.reserved + (uint32_t)M);
+        }
+        staged = staged && !members.empty();
         Factor zero[R], on[R];
         for (int k = 0; k < count; ++k) {
             const FusedOp& m = ops[(size_t)(first + k)];
@@ -623,6 +705,7 @@ struct Gen {
             }
             const int M = m.local >= 0 ? reg_of_local(m.local) : -1;
             if (M >= 0) {
+                if (staged) continue;
                 const std::string c = coef_ptr(om, m), n = std::to_string(uid++);
                 os << "const " << T << " zr" << n << " = (" << T << ")" << c << "[0], zi" << n << " = (" << T << ")" << c
                    << "[1], or" << n << " = (" << T << ")" << c << "[6], oi" << n << " = (" << T << ")" << c << "[7];\n";
@@ -642,6 +725,20 @@ struct Gen {
         Factor u;
         if (any_u) u = {"ur", "ui", false};
         else if (!early.empty()) u = {"hr" + h, "hi" + h, false};
+        if (staged) {
+            os << "{ const V* ph = phases + " << NR * phase_groups.size() << ";\n";
+            for (int i = 0; i < NR; i += 2) {  // two at a time: 16-byte loads
+                os << "{ const float4 v = *reinterpret_cast<const float4*>(ph + " << i << ");\n";
+                for (int j = 0; j < 2; ++j) {
+                    const Factor f = times(u, {j ? "v.z" : "v.x", j ? "v.w" : "v.y", false});
+                    cmul_reg(i + j, f.re.c_str(), f.im.c_str());
+                }
+                os << "}\n";
+            }
+            os << "}\n}\n";
+            phase_groups.push_back(members);
+            return;
+        }
         const size_t half = bits.size() / 2;
         std::vector<Factor> lo(1), hi(1, u);
         for (size_t j = 0; j < bits.size(); ++j) {
@@ -1079,6 +1176,10 @@ struct Gen {
                 }
             }
             resolve(op.reg);
+            if (table_rotation(op)) {
+                rotate_by_table(op);
+                break;
+            }
             const int M = op.reg;
             const int n = open_conditions(op.cmask_outer, tb);
             const std::string c = coef_ptr(o, op);
@@ -1398,7 +1499,7 @@ Fold fold_plan(const Plan& plan, bool across) {
 }
 
 Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, const Fold& fold, int qubits, bool fp64,
-                   Carry* carry, bool last, uint32_t hist_mask = 0, bool zero_start = false) {
+                   Carry* carry, bool last, uint32_t hist_mask = 0, bool zero_start = false, bool table_rotations = false) {
     Gen g;
     g.fp64 = fp64;
     g.K = p.k;
@@ -1504,6 +1605,7 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     os << "FusedOp* prog = reinterpret_cast<FusedOp*>(smem_raw + " << tiles * tile_bytes + hist_bytes << ");\n";
     os << g.T << "* table = reinterpret_cast<" << g.T << "*>(smem_raw + " << (tiles * tile_bytes + hist_bytes + prog_bytes)
        << ");\n";
+    if (tabled && !fp64) os << "V* phases = reinterpret_cast<V*>(table + 8 * P.table_slots);\n(void)phases;\n";
     os << (teams ? "const u32 t = threadIdx.x & " + hexu((uint32_t)nt - 1u) + ";\n" : "const u32 t = threadIdx.x;\n");
     os << "{ const uint2* src = reinterpret_cast<const uint2*>(P.ops); uint2* dst = reinterpret_cast<uint2*>(prog);\n"
        << "  for (int i = threadIdx.x; i < " << p.op_count * (int)(sizeof(FusedOp) / 8) << "; i += " << nt * (teams ? 2 : 1)
@@ -1541,6 +1643,21 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     // complex64 has the registers to keep what depends on the state alone
     std::ostringstream per_state;
     if (tabled && !fp64) g.hoist = &per_state;
+    size_t tabled_ops = 0;
+    for (int o = 0; o < p.op_count; ++o) {
+        const FusedOp& op = plan_ops[(size_t)(p.op_begin + o)];
+        if (!(op.flags & kOpTable)) continue;
+        ++tabled_ops;
+        // up to 192 of them: 2^-96, far from the end of complex64's range
+        if (table_rotations && op.code == OP_MATRIX_REAL && !(op.flags & kOpBranch) && !op.cmask_local && !op.cmask_outer &&
+            g.rotation_slots.size() < 192)
+            g.rotation_slots.push_back(op.reserved);
+    }
+    if (g.rotation_slots.size() > 1) {
+        g.scaled_slot = (int)g.rotation_slots.back();
+        g.rotation_slots.pop_back();
+    }
+    if (table_rotations && !fp64) g.phase_room = 4 * tabled_ops / NR;  // 32 spare bytes a row
     if (tabled) os << kPerStateVars;
     if (hist) {
         os << "for (long long u = blockIdx.x; u < total / " << chunk << "; u += gridDim.x) {\n";
@@ -1724,6 +1841,7 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
         hd << "__device__ __forceinline__ u32 qm_swz(u32 j) { const u32 h = j >> 4; return j ^ ((h ^ (h >> 4) ^ (h >> 8)) "
               "& 15u); }\n";
     const size_t na = std::max<size_t>(1, g.aux.size());
+    const std::string staging = g.state_tables(nt, hd);
     hd << "struct Aux { " << g.T << " v[" << na << "]; };\n";
     hd << "extern \"C\" __global__ void __launch_bounds__(" << nt * (teams ? 2 : 1) << ", " << minb
        << ") qm_pass(V* __restrict__ s0, const __grid_constant__ FusedLaunch P, const __grid_constant__ Aux A"
@@ -1737,7 +1855,7 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
         if (at != std::string::npos) out.src.replace(at, std::strlen(mark), code);
     };
     place(kPerStateVars, g.hoisted);
-    place(kPerState, per_state.str());
+    place(kPerState, staging + per_state.str());
     out.tiles = tiles;
     out.teams = teams ? 2 : 1;
     out.hist_bins = hist_bins;
@@ -1767,7 +1885,7 @@ std::vector<Generated> generate_plan(const Plan& plan, bool chained) {
     for (size_t i = 0; i < plan.passes.size(); ++i)
         out.push_back(generate(plan.passes[i], plan.ops, fold, plan.qubits, fp64, chained ? &carry : nullptr,
                                i + 1 == plan.passes.size(), i + 1 == plan.passes.size() ? plan.hist_mask : 0u,
-                               i == 0 && plan.start_zero));
+                               i == 0 && plan.start_zero, plan.table_rotations));
     return out;
 }
 
