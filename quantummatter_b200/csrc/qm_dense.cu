@@ -407,13 +407,13 @@ bool tile_map_dims(uint32_t tile_mask, int qubits, int32_t* lo, int32_t* len, in
     return r > 0 && tile[0] == 1;
 }
 
-bool encode_tile_map(CUtensorMap* map, void* amps, int precision, int rank, const int32_t* lo, const int32_t* len,
+bool encode_tile_map(CUtensorMap* map, void* amps, int rank, const int32_t* lo, const int32_t* len,
                      const int32_t* tile) {
     auto encode = tensor_map_encoder();
     if (!encode || rank < 1 || rank > kDenseTmaMaxRank) return false;
     cuuint64_t dims[kDenseTmaMaxRank], strides[kDenseTmaMaxRank];
     cuuint32_t box[kDenseTmaMaxRank], estr[kDenseTmaMaxRank];
-    const int elem = precision == QM_FP32 ? 8 : 16;
+    const int elem = 8;  // complex64
     for (int d = 0; d < rank; ++d) {
         dims[d] = (cuuint64_t)1 << len[d];
         box[d] = tile[d] ? (cuuint32_t)1 << len[d] : 1u;
@@ -422,16 +422,16 @@ bool encode_tile_map(CUtensorMap* map, void* amps, int precision, int rank, cons
     }
     dims[0] *= 2;  // the innermost dimension counts scalars: (re, im) pairs
     box[0] *= 2;
-    return encode(map, precision == QM_FP32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                   (cuuint32_t)rank, amps, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool dense_geometry(int qubits, int precision, const DenseOp& op, DenseGeometry& g) {
+bool dense_geometry(int qubits, const DenseOp& op, DenseGeometry& g) {
     const int m = op.m;
     if (m < 1 || m > kDenseMaxQubits || qubits < 9) return false;
-    const int elem = precision == QM_FP32 ? 8 : 16;
+    const int elem = 8;  // complex64
     uint32_t qmask = 0;
     for (int i = 0; i < m; ++i) qmask |= 1u << op.q[i];
     const int tb = std::min(kDenseTileBits, qubits);
@@ -460,14 +460,13 @@ bool dense_geometry(int qubits, int precision, const DenseOp& op, DenseGeometry&
     g.copies = 1 << (tb - r);
     const int run_bytes = elem << r;
     // A tensor-map box is the unpadded natural order, whose column accesses are free of bank
-    // conflicts when the lowest index bits (a wavefront's worth: 8 complex128, 16 complex64) are
-    // column bits; otherwise only 1- and 2-qubit gates (too little arithmetic to mind) take it.
+    // conflicts when the lowest index bits (a wavefront's worth: 16 amplitudes) are column bits.
     g.tma_rank = 0;
     {
-        const int low = precision == QM_FP32 ? 4 : 3;
+        const int low = 4;
         const bool contiguous_columns = (lmask & ((1u << low) - 1u)) == ((1u << low) - 1u);
         int32_t rank = 0;
-        if (dense_tma_enabled() && (contiguous_columns || m <= 2) &&
+        if (dense_tma_enabled() && contiguous_columns &&
             tile_map_dims(qmask | lmask, qubits, g.tma_lo, g.tma_len, g.tma_tile, &rank))
             g.tma_rank = rank;
     }
@@ -512,7 +511,7 @@ cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& o
         return cudaGetLastError();
     }
     DenseGeometry g;
-    if (!dense_geometry(qubits, precision, op, g)) return cudaErrorInvalidValue;
+    if (!dense_geometry(qubits, op, g)) return cudaErrorInvalidValue;
     DenseLaunch P{};
     P.matrix = matrix;
     P.status = status;
@@ -532,7 +531,7 @@ cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& o
     P.m = op.m;
     P.tma_rank = 0;
     if (g.tma_rank) {
-        if (encode_tile_map(&P.tmap, amps, precision, g.tma_rank, g.tma_lo, g.tma_len, g.tma_tile)) {
+        if (encode_tile_map(&P.tmap, amps, g.tma_rank, g.tma_lo, g.tma_len, g.tma_tile)) {
             P.tma_rank = g.tma_rank;
             for (int d = 0; d < g.tma_rank; ++d) {
                 P.tma_lo[d] = g.tma_lo[d];

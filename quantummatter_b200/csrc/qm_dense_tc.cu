@@ -616,7 +616,7 @@ cudaError_t launch_dense_tc(void* amps, int qubits, const DenseOp& op, const flo
     P.tile_mask = qmask | lmask;
     int32_t rank = 0;
     if (dense_tma_enabled() && tile_map_dims(P.tile_mask, qubits, P.tma_lo, P.tma_len, P.tma_tile, &rank) &&
-        encode_tile_map(&P.tmap, amps, QM_FP32, rank, P.tma_lo, P.tma_len, P.tma_tile))
+        encode_tile_map(&P.tmap, amps, rank, P.tma_lo, P.tma_len, P.tma_tile))
         P.tma_rank = rank;
     for (int b = 0, local = 0; b < qubits; ++b) {
         if (!((P.tile_mask >> b) & 1u)) continue;

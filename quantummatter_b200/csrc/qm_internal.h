@@ -196,7 +196,7 @@ int default_block_qubits(int qubits, int precision);
 // Dense fused gates of at most `width` (1..6) qubits (qm_dense.cpp).
 bool plan_dense(const std::vector<qm_gate>& gates, int qubits, int precision, int width, Plan& plan,
                 std::string& error);
-bool dense_geometry(int qubits, int precision, const DenseOp& op, DenseGeometry& g);
+bool dense_geometry(int qubits, const DenseOp& op, DenseGeometry& g);
 // Tiles of dense fused gates move as tensor-map boxes (cp.async.bulk.tensor) where their bit runs
 // form at most five dimensions; QM_DENSE_TMA=0 keeps them on plain copies.
 constexpr int kDenseTmaMaxRank = 5;
@@ -205,7 +205,7 @@ bool dense_tma_enabled();
 // they need more than five.  encode_tile_map builds the map over the state at `amps` (tile runs at
 // full extent in the box, outer runs at extent 1); false without the driver's encoder.
 bool tile_map_dims(uint32_t tile_mask, int qubits, int32_t* lo, int32_t* len, int32_t* tile, int32_t* rank);
-bool encode_tile_map(CUtensorMap* map, void* amps, int precision, int rank, const int32_t* lo, const int32_t* len,
+bool encode_tile_map(CUtensorMap* map, void* amps, int rank, const int32_t* lo, const int32_t* len,
                      const int32_t* tile);
 // One dense fused gate on a state (qm_dense.cu); `matrix` is its transposed unitary in device memory.
 cudaError_t launch_dense(void* amps, int qubits, int precision, const DenseOp& op, const double* host_matrix,
