@@ -343,6 +343,7 @@ constexpr const char* kPerStateVars = "/*vars*/";
 struct Gen {
     std::ostringstream os;
     bool fp64;
+    bool packed = false;  // two parts of an amplitude in one multiply-add (qm_fma2)
     int K;
     int phys[NR];
     uint32_t pm[R];  // local masks of the register bits in the current layout
@@ -428,7 +429,7 @@ struct Gen {
             const int k = i | (1 << M);
             os << "{ const " << T << " xr = " << X(i) << ", xi = " << Y(i) << ", yr = " << X(k) << ", yi = " << Y(k)
                << ";\n";
-            if (real && !fp64) {
+            if (real && packed) {
                 os << "float ur, ui, vr, vi; qm_mul2(ur, ui, br, yr, yi); qm_mul2(vr, vi, dr, yr, yi);\n";
                 os << "qm_fma2(" << X(i) << ", " << Y(i) << ", ar, xr, xi, ur, ui); qm_fma2(" << X(k) << ", " << Y(k)
                    << ", cr, xr, xi, vr, vi); }\n";
@@ -1099,7 +1100,7 @@ struct Gen {
         if (dep_count(q) > kMaxVariantBits) flush_all();
         os << "{\n";
         // complex64: form B takes -w, so that both halves of a packed multiply-add have one sign
-        const bool packed = !fp64, minus = packed && sp.form_b;
+        const bool minus = packed && sp.form_b;
         PairPhase P = take_phase(q, sp.lam, true);
         if (minus && P.cls < 2) P.cls ^= 1;
         for (int i = 0; minus && i < NR; ++i) P.quad[i] ^= 2;
@@ -1532,6 +1533,10 @@ Generated generate(const FusedPass& p, const std::vector<FusedOp>& plan_ops, con
     bool tabled = false;
     for (int o = 0; o < p.op_count; ++o)
         if (plan_ops[(size_t)(p.op_begin + o)].flags & kOpTable) tabled = true;
+    // Packed multiply-adds pay where issue slots bind: depth 20 at 24 qubits 1574 to 1551 us, at 25 3363 to
+    // 3217, at 27 12.9 to 11.95 ms; at 20 to 22 qubits, a wave or a few of tiles, 1 to 5 % slower (depth 7:
+    // 160 to 167 us at 22, 582 to 587 at 24).  The results are the same to the bit.
+    g.packed = !fp64 && (tabled || qubits >= 25);
     // The tile pipeline needs a second tile of shared memory.  Complex64 blocks of 12 qubits keep
     // two blocks per SM with it (5.9 against 6.5 ms per 30-qubit brick pass).  A complex128 block
     // would take an SM alone, and one 8-warp block per SM computes too slowly (12.3 against

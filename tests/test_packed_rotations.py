@@ -10,7 +10,7 @@ import pytest
 
 import oracle as orc
 from circuits import random_state
-from quantummatter_b200.backend import FP32, DeviceState, Plan
+from quantummatter_b200.backend import FP32, FP64, DeviceState, Plan
 from quantummatter_b200.circuit import QuantumCircuit, u3
 
 pytestmark = pytest.mark.gpu
@@ -33,10 +33,19 @@ def circuit(n: int, angle: float) -> QuantumCircuit:
     return c
 
 
-@pytest.mark.parametrize("n", [9, 12, 16])
+@pytest.mark.parametrize("n", [9, 12, 16, 25])
 @pytest.mark.parametrize("angle", [0.2, math.pi / 2, 2.9, math.pi])
 def test_packed_rotations_match_the_oracle(gpu_context, n, angle):
     c, psi = circuit(n, angle), random_state(n, n)
+    if n < 25:
+        want = orc.execute(c, psi)
+    else:  # from 25 qubits on the packed form runs; the complex128 plan in the oracle's place
+        wide = Plan(gpu_context, c, FP64, 0)
+        with DeviceState(gpu_context, n, FP64) as st:
+            st.Upload(psi)
+            wide.execute(st)
+            want = st.Download()
+        wide.Dispose()
     p = Plan(gpu_context, c, FP32, 0)
     with DeviceState(gpu_context, n, FP32) as st:
         st.Upload(psi)
@@ -44,4 +53,4 @@ def test_packed_rotations_match_the_oracle(gpu_context, n, angle):
         got = st.Download()
     p.Dispose()
     # about 300 gates, a few roundings of 6e-8 each on amplitudes of at most 1
-    assert np.max(np.abs(got - orc.execute(c, psi))) <= 2e-5
+    assert np.max(np.abs(got - want)) <= 2e-5
