@@ -336,7 +336,18 @@ int32_t build_plan(qm_context* ctx, int32_t qubits, int32_t precision, const qm_
     // structures; they never wait for a compilation.  Below 26 qubits a pass takes well under a
     // millisecond, about what generating the plan's sources for the lookup costs on the host,
     // so those run the interpreter.
-    if (transient && qubits >= 26) jit_lookup(plan);
+    if (transient && qubits >= 26) {
+        jit_lookup(plan);
+        // none there: the interpreter's form of the circuit (27 qubits, complex64,
+        // depth 38: 130 ms with the circuit as given, 109 so)
+        const bool found = std::any_of(plan.jit.begin(), plan.jit.end(), [](const void* k) { return k != nullptr; });
+        if (!found && (width == 0 || width >= 9)) {
+            Plan again;
+            if (!plan_fused(one_shot_gates(list, precision), qubits, precision, width, again, err))
+                return fail(QM_E_ARG, "planner: " + err);
+            plan = std::move(again);
+        }
+    }
     if (transient) return plan_upload(plan, ctx->stream, &ctx->program, &ctx->program_bytes);
     return plan_upload(plan, ctx->stream);
 }

@@ -10,7 +10,7 @@ import pytest
 
 import oracle as orc
 from circuits import random_circuit, random_state
-from quantummatter_b200.backend import FP32, FP64, DeviceState
+from quantummatter_b200.backend import FP32, FP64, DeviceState, Plan
 from quantummatter_b200.circuit import QuantumCircuit, SingleQubitUnitary, u3
 from quantummatter_b200.workloads import brick_circuit
 
@@ -45,3 +45,19 @@ def test_one_shot_circuits_match_the_oracle(gpu_context, n, precision, tol):
                 got = st.Download()
             assert np.max(np.abs(got - want)) <= tol, width
             assert abs(np.sum(np.abs(got) ** 2) - np.sum(np.abs(psi) ** 2)) <= 50 * tol
+
+
+@pytest.mark.parametrize("precision,tol", [(FP64, 5e-13), (FP32, 2e-6)], ids=["fp64", "fp32"])
+def test_large_states_without_compiled_passes(gpu_context, precision, tol):
+    """26 qubits, no kernel of the circuit's structure compiled yet: the interpreter's form of the circuit
+    against the compiled plan (amplitudes of about 1e-4, tolerances of 1e-2 of them and less)."""
+    n, c = 26, brick_circuit(26, 5, seed=61)
+    with DeviceState(gpu_context, n, precision) as st:
+        st.Evolve(c)
+        got = st.Download()
+    p = Plan(gpu_context, c, FP64, 0)
+    with DeviceState(gpu_context, n, FP64) as st:
+        p.execute(st)
+        want = st.Download()
+    p.Dispose()
+    assert np.max(np.abs(got - want)) <= tol
