@@ -1323,11 +1323,13 @@ int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t cou
     plan_pauli_sum(st->qubits, st->precision, terms, count, ctx->sm_count, plan);
     const size_t program = pauli_sum_inline(plan) ? 0 : (plan.program.size() + 255) & ~size_t(255);
     const size_t masses = (size_t)plan.parts * plan.tiles, cells = (size_t)plan.grid * plan.columns;
-    int32_t rc = ensure_scratch(ctx, program + sizeof(double) * (masses + cells + plan.columns));
+    const size_t folds = pauli_sum_folds(plan);
+    int32_t rc = ensure_scratch(ctx, program + folds + sizeof(double) * (masses + cells + plan.columns));
     if (rc) return rc;
     rc = ensure_host_scratch(ctx, program + sizeof(double) * plan.columns);
     if (rc) return rc;
-    double* tile_masses = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + program);
+    double2* fold = reinterpret_cast<double2*>(static_cast<char*>(ctx->scratch) + program);
+    double* tile_masses = reinterpret_cast<double*>(reinterpret_cast<char*>(fold) + folds);
     double* partials = tile_masses + masses;
     double* out = partials + cells;
     double* host = ctx->host_scratch + program / sizeof(double);
@@ -1336,7 +1338,7 @@ int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t cou
         QM_CUDA(cudaMemcpyAsync(ctx->scratch, ctx->host_scratch, plan.program.size(), cudaMemcpyHostToDevice, ctx->stream));
     }
     QM_CUDA(launch_pauli_sum(st->amps, st->precision, plan, program ? ctx->scratch : nullptr, tile_masses, partials,
-                             ctx->stream));
+                             fold, ctx->stream));
     QM_CUDA(launch_finish_sums(partials, (int)plan.grid, plan.columns, out, ctx->stream));
     QM_CUDA(cudaMemcpyAsync(host, out, sizeof(double) * plan.columns, cudaMemcpyDeviceToHost, ctx->stream));
     QM_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -343,9 +343,11 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
 // Whether the plan's program fits the kernels' parameters (launch_pauli_sum then takes no copy of it).
 bool pauli_sum_inline(const PauliSumPlan& plan);
 // Partial sums [grid][columns] of every term but the wide ones, the mass in the last column;
-// tile_masses holds parts * tiles doubles, `program` the plan's program in device memory or null.
+// tile_masses holds parts * tiles doubles, folds pauli_sum_folds bytes, `program` the plan's program in
+// device memory or null.
+size_t pauli_sum_folds(const PauliSumPlan& plan);
 cudaError_t launch_pauli_sum(const void* amps, int precision, const PauliSumPlan& plan, const void* program,
-                             double* tile_masses, double* partials, cudaStream_t s);
+                             double* tile_masses, double* partials, double2* folds, cudaStream_t s);
 
 // ---------------------------------------------------------------- tiled expectation (qm_expect.cu)
 constexpr int kTileMaxTerms = 256;

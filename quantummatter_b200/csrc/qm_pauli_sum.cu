@@ -13,18 +13,23 @@
 //   signs sums to zero.  Between stages the tile is read again from shared memory (16-byte slots
 //   XORed with higher index bits, free of bank conflicts); a stage on the four highest tile qubits
 //   uses the registers as loaded.  Each thread keeps a running sum per term in shared memory, so a
-//   warp reduces once per block and not once per tile and term.
+//   warp reduces once per twelve tiles and not once per tile and term.
 // - Diagonal terms.  Signs on tile qubits only: every thread sums its 16 probabilities over its
 //   tiles, and one Walsh-Hadamard transform per block at the end gives every such term.  Signs on
 //   outer qubits too: the tile's signed mass for each distinct tile part is written per tile, and
 //   k_outer_terms sums those with the signs of the tile index.
 // Products and sums are FP64 for both precisions (complex64 amplitudes widen when they are loaded).
+// No value goes through more plain additions than in a reduction of every tile by itself (19 for a
+// flip's pairs: 7 in a thread, 5 in a warp, 7 over warps; 12 in a tile's transform).  A running sum is
+// closed after twelve tiles (3 + 11 + 3 additions, 11 for a probability) and what follows carries its
+// rounding errors along.  Left plain until the block's end, a sum over its 222 tiles at 28 qubits was
+// 4 % faster.
 //
 // Bound: 28 qubits complex128, XXZ chain of 109 terms: three passes of 0.67 ms of HBM, 1.0 ms of FP64,
 // about 2 ms of shared-memory wavefronts; 16 warps per SM wait on shared loads between them.  With
 // pairs read from shared memory and a warp reduction per term and tile the same call took 23.3 ms,
-// 8.4 of them to add up 2^18 rows; 5.5 ms now (10 qubits: 57 to 46 us).  Two blocks per SM set the pass's 22 running sums (the
-// 11 bonds of a 12-qubit tile); 11-qubit tiles need a fourth pass.
+// 8.4 of them to add up 2^18 rows; 5.7 ms now (10 qubits: 57 to 46 us).  Two blocks per SM set the pass's
+// 22 running sums (the 11 bonds of a 12-qubit tile); 11-qubit tiles need a fourth pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,6 +50,7 @@ constexpr int kThreads = 1 << (kMaxTile - 4);
 constexpr int kEntries = 11;    // pairs of running sums per thread (terms that flip qubits) and pass: two blocks per SM
 constexpr int kMaxParts = 16;   // distinct tile parts of diagonal terms with outer signs, per pass
 constexpr int kOuterRows = 16;  // partial rows of k_outer_terms at most
+constexpr uint32_t kFoldTiles = 12;  // tiles of a block between two compensated additions
 
 struct SumEntry {           // one or two terms with one flip mask, both real parts or both imaginary
     double sign[2][3];      // +-1 of the pair index's bits
@@ -80,9 +86,11 @@ struct SumPass {
     uint32_t tile_mask, outer_mask;
     int32_t stage, stages, entry, entries, part, parts;
     int32_t direct;         // whether the first stage is the load layout
-    int32_t pad[3];
+    uint32_t reg_at[4];     // index bits of the load layout's register bits
+    uint32_t step_at;       // from a block's tile to its next: index bits of the grid size
+    int32_t pad[2];
 };
-static_assert(sizeof(SumEntry) == 96 && sizeof(SumPart) == 40 && sizeof(SumStage) == 32 && sizeof(SumPass) == 48,
+static_assert(sizeof(SumEntry) == 96 && sizeof(SumPart) == 40 && sizeof(SumStage) == 32 && sizeof(SumPass) == 64,
               "device layout");
 
 // Programs up to this size travel as kernel parameters, which saves small states a copy.
@@ -97,6 +105,7 @@ struct SumLaunch {
     uint32_t tiles;
     double* tile_masses;           // [part][tiles]
     double* partials;              // [rows][columns]
+    double2* folds;                // [grid][kRegs][threads]: probabilities of more than kFoldTiles tiles
     __align__(16) unsigned char inline_program[kInlineProgram];
     template <typename V>
     __device__ __forceinline__ const V* list(int i) const {
@@ -167,11 +176,20 @@ __device__ __forceinline__ void run_stage(const double2 (&x)[kRegs], int first, 
 }
 
 __host__ __device__ constexpr size_t program_bytes() {
-    return sizeof(SumPass) + kEntries * (sizeof(SumStage) + sizeof(SumEntry) + sizeof(double2)) +
+    return sizeof(SumPass) + kEntries * (sizeof(SumStage) + sizeof(SumEntry) + sizeof(double2) + 2 * sizeof(KSum)) +
            kMaxParts * (sizeof(SumPart) + 8 * sizeof(double));
 }
 
-// Shared memory: [tile: 2^k double2][pass program][warp sums of parts][outer signs][running sums]
+// x + y and x - y of two sums that carry their rounding errors in .y.
+__device__ __forceinline__ void butterfly(double2& x, double2& y) {
+    const double s = x.x + y.x, sb = s - x.x, se = (x.x - (s - sb)) + (y.x - sb);
+    const double d = x.x - y.x, db = d - x.x, de = (x.x - (d - db)) - (y.x + db);
+    const double a = x.y, b = y.y;
+    x = make_double2(s, se + (a + b));
+    y = make_double2(d, de + (a - b));
+}
+
+// Shared memory: [tile: 2^k double2][pass program][warp sums of parts][totals][outer signs][running sums]
 template <typename T, bool DIAG>
 __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T>::type* __restrict__ s,
                                                            const __grid_constant__ SumLaunch L) {
@@ -191,7 +209,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
     double2* outer_sign = reinterpret_cast<double2*>(entries + pass->entries);  // [entries], of the current tile
     SumPart* parts = reinterpret_cast<SumPart*>(outer_sign + pass->entries);
     double* warp_part = reinterpret_cast<double*>(parts + pass->parts);  // [parts][8]
-    double* sums = warp_part + 8 * pass->parts;                          // [2 entries][nt]
+    KSum* totals = reinterpret_cast<KSum*>(warp_part + 8 * pass->parts);  // [2 entries]
+    double* sums = reinterpret_cast<double*>(totals + 2 * pass->entries);  // [2 entries][nt]
     auto copy = [&](void* dst, const void* from, size_t bytes) {
         for (uint32_t i = t; i < bytes / 4; i += nt)
             reinterpret_cast<uint32_t*>(dst)[i] = reinterpret_cast<const uint32_t*>(from)[i];
@@ -201,20 +220,38 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
     copy(parts, L.list<SumPart>(3) + pass->part, sizeof(SumPart) * pass->parts);
     double* acc = sums + t;
     for (int i = 0; i < 2 * pass->entries; ++i) acc[(size_t)i * nt] = 0.0;
+    if (t < 2u * pass->entries) totals[t] = KSum{0.0, 0.0};
+    if (DIAG)
+        for (uint32_t i = t; i < 8u * pass->parts; i += nt) warp_part[i] = 0.0;  // tiles of fewer than eight warps
     __syncthreads();
 
-    const uint32_t outer_mask = pass->outer_mask;
     // the load layout: threads on the lowest k - 4 tile bits, registers on the four highest
     const uint32_t thread_at = deposit(t, pass->tile_mask);
-    uint32_t reg_at[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) reg_at[m] = deposit(nt << m, pass->tile_mask);
-    const uint32_t step_at = deposit(gridDim.x, outer_mask);
-    uint32_t outer = deposit(blockIdx.x, outer_mask);
+    uint32_t outer = deposit(blockIdx.x, pass->outer_mask);
     double prob[DIAG ? kRegs : 1];
 #pragma unroll
     for (int i = 0; i < (DIAG ? kRegs : 1); ++i) prob[i] = 0.0;
 
+    uint32_t done = 0;  // tiles of this block
+    // the threads' running sums into the block's compensated totals, each sum by one warp
+    auto fold = [&]() {
+        for (uint32_t i = warp; i < 2u * pass->entries; i += warps) {
+            const uint32_t mask = entries[i >> 1].thread_mask[i & 1];
+            double v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t c = lane + 32 * j;
+                v[j] = 0.0;
+                if (c < nt) {
+                    v[j] = signed_if(sums[(size_t)i * nt + c], (uint32_t)__popc(c & mask) & 1u);
+                    sums[(size_t)i * nt + c] = 0.0;
+                }
+            }
+            KSum w{((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])), 0.0};
+            for (int d = 16; d > 0; d >>= 1) w.merge(shfl_down_ksum(w, d));
+            if (lane == 0) totals[i].merge(w);
+        }
+    };
     for (uint32_t item = blockIdx.x; item < L.tiles; item += gridDim.x) {
         double2 x[kRegs];
 #pragma unroll
@@ -222,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
             uint32_t g = outer | thread_at;
 #pragma unroll
             for (int m = 0; m < 4; ++m)
-                if ((i >> m) & 1) g |= reg_at[m];
+                if ((i >> m) & 1) g |= pass->reg_at[m];
             const Cx<T> v = load_amp<T>(s, g);
             x[i] = make_double2((double)v.re, (double)v.im);
         }
@@ -252,9 +289,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
             reinterpret_cast<double*>(outer_sign)[t] = (__popc(outer & entries[t >> 1].outer_mask[t & 1]) & 1) ? -1.0 : 1.0;
         __syncthreads();  // the tile, the warps' parts and the signs are in shared memory
         if (DIAG && t < (uint32_t)pass->parts) {
-            double w = 0.0;
-            for (uint32_t i = 0; i < warps; ++i) w += warp_part[8 * t + i];
-            L.tile_masses[(size_t)parts[t].index * L.tiles + item] = w;
+            const double* w = warp_part + 8 * t;
+            L.tile_masses[(size_t)parts[t].index * L.tiles + item] =
+                ((w[0] + w[1]) + (w[2] + w[3])) + ((w[4] + w[5]) + (w[6] + w[7]));
         }
 #pragma unroll 1
         for (int st = 0; st < pass->stages; ++st) {
@@ -279,21 +316,61 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
             run_stage(x, stage.entry, stage.entries, entries, outer_sign, acc, nt);
         }
         __syncthreads();  // every read of the tile is done
-        outer = deposit_add(outer, step_at, outer_mask);
+        outer = deposit_add(outer, pass->step_at, pass->outer_mask);
+        if (++done % kFoldTiles == 0 && item + gridDim.x < L.tiles) {
+            fold();
+            if (DIAG && L.pass + blockIdx.y == 0) {
+                double2* folds = L.folds + ((size_t)blockIdx.x * kRegs * nt + t);
+#pragma unroll
+                for (int i = 0; i < kRegs; ++i) {
+                    const double2 f = done > kFoldTiles ? folds[nt * i] : make_double2(0.0, 0.0);
+                    KSum sum{f.x, f.y};
+                    sum.add(prob[i]);
+                    folds[nt * i] = make_double2(sum.s, sum.c);
+                    prob[i] = 0.0;
+                }
+            }
+            __syncthreads();
+        }
     }
 
     // one row of sums per block; a pair's two members contribute the same
+    fold();
     for (uint32_t i = warp; i < 2u * pass->entries; i += warps) {
         const SumEntry& e = entries[i >> 1];
         if ((i & 1) && !e.both) continue;
-        double w = 0.0;
-        for (uint32_t c = lane; c < nt; c += 32)
-            w += signed_if(sums[(size_t)i * nt + c], (uint32_t)__popc(c & e.thread_mask[i & 1]) & 1u);
-        w = warp_total(w);
-        if (lane == 0) row[e.column[i & 1]] = e.negate[i & 1] ? -2.0 * w : 2.0 * w;
+        if (lane == 0) row[e.column[i & 1]] = e.negate[i & 1] ? -2.0 * totals[i].value() : 2.0 * totals[i].value();
     }
     if (DIAG && L.pass + blockIdx.y == 0) {
-        // Walsh-Hadamard transform of the summed probabilities over the tile's bits
+        // Walsh-Hadamard transform of the summed probabilities over the tile's bits: with the rounding
+        // errors of a block's sums over several tiles, plainly for one tile
+        const SumLocal* locals = L.list<SumLocal>(4);
+        if (L.tiles > gridDim.x) {
+            const double2* folds = L.folds + ((size_t)blockIdx.x * kRegs * nt + t);
+#pragma unroll
+            for (int i = 0; i < kRegs; ++i) {
+                KSum sum{prob[i], 0.0};
+                if (done > kFoldTiles) {
+                    const double2 f = folds[nt * i];
+                    sum = KSum{f.x, f.y};
+                    sum.add(prob[i]);
+                }
+                tile[t + nt * i] = make_double2(sum.s, sum.c);
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int m = 0; m < k; ++m) {
+#pragma unroll 1
+                for (uint32_t i = t; i < (kRegs / 2) * nt; i += nt) {
+                    const uint32_t j = insert_zero(i, m);
+                    butterfly(tile[j], tile[j | (1u << m)]);
+                }
+                __syncthreads();
+            }
+            for (int i = t; i < L.local_count; i += nt)
+                row[locals[i].column] = locals[i].factor * (tile[locals[i].mask].x + tile[locals[i].mask].y);
+            return;
+        }
         double* w = reinterpret_cast<double*>(smem);
 #pragma unroll
         for (int m = 0; m < 4; ++m)
@@ -316,7 +393,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
             }
             __syncthreads();
         }
-        const SumLocal* locals = L.list<SumLocal>(4);
         for (int i = t; i < L.local_count; i += nt) row[locals[i].column] = locals[i].factor * w[locals[i].mask];
     }
 }
@@ -448,6 +524,13 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
         SumPass p{};
         p.tile_mask = Q;
         p.outer_mask = all & ~Q;
+        for (int q = 0, b = 0; q < qubits; ++q)
+            if ((Q >> q) & 1u) {
+                if (b >= regs_at) p.reg_at[b - regs_at] = 1u << q;
+                ++b;
+            }
+        for (int q = 0, b = 0; q < qubits; ++q)
+            if ((p.outer_mask >> q) & 1u) p.step_at |= ((plan.grid >> b++) & 1u) << q;
         p.stage = (int32_t)stages.size();
         p.entry = (int32_t)entries.size();
         p.part = (int32_t)parts.size();
@@ -530,10 +613,15 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
     plan.at[5] = append(plan.program, outers);
 }
 
+size_t pauli_sum_folds(const PauliSumPlan& plan) {
+    const bool long_runs = (uint64_t)plan.tiles > (uint64_t)kFoldTiles * plan.grid;
+    return long_runs ? sizeof(double2) * ((size_t)plan.grid << plan.k) : 0;
+}
+
 bool pauli_sum_inline(const PauliSumPlan& plan) { return plan.program.size() <= (size_t)kInlineProgram; }
 
 cudaError_t launch_pauli_sum(const void* amps, int precision, const PauliSumPlan& plan, const void* program,
-                             double* tile_masses, double* partials, cudaStream_t st) {
+                             double* tile_masses, double* partials, double2* folds, cudaStream_t st) {
     SumLaunch L;
     L.program = static_cast<const unsigned char*>(program);
     if (!program) std::memcpy(L.inline_program, plan.program.data(), plan.program.size());
@@ -543,6 +631,7 @@ cudaError_t launch_pauli_sum(const void* amps, int precision, const PauliSumPlan
     L.tiles = plan.tiles;
     L.tile_masses = tile_masses;
     L.partials = partials;
+    L.folds = folds;
     cudaError_t e = cudaSuccess;
     L.pass = 0;
     L.local_count = plan.locals;
