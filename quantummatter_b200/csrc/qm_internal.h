@@ -61,6 +61,11 @@ constexpr int kMaxPassOps = 256;    // ops per pass: the program (88 B per op) i
 constexpr int kMaxPassGates = 120;  // gates absorbed per pass (stage changes add at most gates + 2)
 
 constexpr uint16_t kOpTable = 4;    // FusedOp::flags: coefficients come from the batch's table
+// OP_DIAG by one constant phase, 1 where the target is 0: coef[kCoefTurn] holds its angle as a whole
+// number of 2^-64 turns (the bits of a uint64_t), coef[kCoefExcess] its modulus less 1.  Both lie in the
+// half of the coefficients that the interpreting kernel's conversion to the state's precision leaves.
+constexpr uint16_t kOpTurn = 32;
+constexpr int kCoefTurn = 4, kCoefExcess = 5;
 constexpr uint16_t kOpRotation = 16;  // set by the interpreting kernel on its own copy of a program: see k_fused
 constexpr uint16_t kOpBranch = 8;   // FusedOp::flags: a table op realising a noise branch; the kernel
                                     // skips identities and applies real diagonals as scalings

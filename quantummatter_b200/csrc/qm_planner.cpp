@@ -73,6 +73,18 @@ GInfo classify(const qm_gate& g, int32_t slot) {
 
 inline bool blocked(const GInfo& g, uint32_t bx, uint32_t bz) { return (g.touch & bx) || (g.xmask & bz); }
 
+// Marks a phase (a == 1) of modulus 1 to rounding as a turn; moduli of a run add up to first order.
+void set_turn(FusedOp& op) {
+    const long double re = op.coef[6], im = op.coef[7], excess = (re * re + im * im - 1) / 2;
+    if (!(fabsl(excess) <= 1e-12L)) return;
+    long double turns = atan2l(im, re) * 0.159154943091895335768883763372514362L;  // 1 / (2 pi)
+    if (turns < 0) turns += 1;
+    const uint64_t whole = turns < 1 ? (uint64_t)ldexpl(turns, 64) : 0;
+    std::memcpy(&op.coef[kCoefTurn], &whole, sizeof whole);
+    op.coef[kCoefExcess] = (double)excess;
+    op.flags |= kOpTurn;
+}
+
 // a gate's qubits renamed by a permutation of the index bits
 void remap_gate(GInfo& gi, const int* perm) {
     PlanGate& g = gi.g;
@@ -412,6 +424,7 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
                             op.local = (int8_t)lt;
                             op.target_outer = lt >= 0 ? 0u : (1u << g.target);
                             op.flags = (uint16_t)((a1 ? 1 : 0) | (d1 ? 2 : 0));
+                            if (a1) set_turn(op);
                         }
                     } else if (g.kernel == QM_KERNEL_EXCHANGE) {
                         op.code = OP_EXCHANGE;
