@@ -595,7 +595,8 @@ __host__ __device__ constexpr size_t program_bytes(int ops) { return ((size_t)op
 
 // Persistent: each CTA loops over (state, block) work items, so the pass program is staged
 // into shared memory once per CTA and a state's coefficient row once per state change.
-template <typename T, int K>
+// RUNS: the pass holds a run of phases (op_phase_run); its code costs passes without one 4 %.
+template <typename T, int K, bool RUNS>
 __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || (sizeof(T) == 4 && K == 13)) ? 2 : 1)
     k_fused(typename Vec2<T>::type* __restrict__ s0, const __grid_constant__ FusedLaunch P) {
     using V = typename Vec2<T>::type;
@@ -710,7 +711,7 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
                 o += count;
                 continue;
             }
-            if (op.flags & kOpTurn) {
+            if (RUNS && code == OP_DIAG && (op.flags & kOpTurn)) {
                 int count = 1;
                 while (o + count < P.op_count && (prog[o + count].flags & kOpTurn)) ++count;
                 if (count > 1) {
@@ -779,7 +780,7 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
     }
 }
 
-template <typename T, int K>
+template <typename T, int K, bool RUNS>
 cudaError_t launch_k(void* amps, int qubits, const FusedPass& p, const FusedOp* d_ops, const FusedBatch* batch,
                      cudaStream_t st) {
     using V = typename Vec2<T>::type;
@@ -798,19 +799,19 @@ cudaError_t launch_k(void* amps, int qubits, const FusedPass& p, const FusedOp* 
         if (l.err == cudaSuccess) l.err = cudaDeviceGetAttribute(&l.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (l.err == cudaSuccess) l.err = cudaDeviceGetAttribute(&l.sms, cudaDevAttrMultiProcessorCount, dev);
         if (l.err == cudaSuccess)
-            l.err = cudaFuncSetAttribute(k_fused<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, l.optin);
+            l.err = cudaFuncSetAttribute(k_fused<T, K, RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, l.optin);
         return l;
     }();
     if (lim.err != cudaSuccess) return lim.err;
     const int optin = lim.optin, sms = lim.sms;
     if (smem > (size_t)optin) return cudaErrorInvalidValue;  // program or coefficient row too large
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<T, K>, 1 << (K - R), smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<T, K, RUNS>, 1 << (K - R), smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int64_t items = (int64_t)L.states << L.cta_shift;
     const int64_t grid = std::min<int64_t>(items, (int64_t)sms * per_sm);
-    k_fused<T, K><<<(unsigned)grid, 1 << (K - R), smem, st>>>(reinterpret_cast<V*>(amps), L);
+    k_fused<T, K, RUNS><<<(unsigned)grid, 1 << (K - R), smem, st>>>(reinterpret_cast<V*>(amps), L);
     return cudaGetLastError();
 }
 
@@ -849,27 +850,36 @@ FusedLaunch fused_launch_params(int qubits, const FusedPass& p, const FusedOp* d
     return L;
 }
 
-cudaError_t launch_fused(void* amps, int qubits, int precision, const FusedPass& p, const FusedOp* d_ops,
-                         const FusedBatch* batch, cudaStream_t st) {
-    if (p.k > qubits || p.op_count > kMaxPassOps || p.op_count < 0 || !d_ops) return cudaErrorInvalidValue;
-    if (batch && (batch->states < 1 || batch->states > 65535)) return cudaErrorInvalidValue;
+template <bool RUNS>
+static cudaError_t launch_fused_t(void* amps, int qubits, int precision, const FusedPass& p, const FusedOp* d_ops,
+                                  const FusedBatch* batch, cudaStream_t st) {
     if (precision == QM_FP32) {
         switch (p.k) {
-        case 9: return launch_k<float, 9>(amps, qubits, p, d_ops, batch, st);
-        case 10: return launch_k<float, 10>(amps, qubits, p, d_ops, batch, st);
-        case 11: return launch_k<float, 11>(amps, qubits, p, d_ops, batch, st);
-        case 12: return launch_k<float, 12>(amps, qubits, p, d_ops, batch, st);
-        case 13: return launch_k<float, 13>(amps, qubits, p, d_ops, batch, st);
+        case 9: return launch_k<float, 9, RUNS>(amps, qubits, p, d_ops, batch, st);
+        case 10: return launch_k<float, 10, RUNS>(amps, qubits, p, d_ops, batch, st);
+        case 11: return launch_k<float, 11, RUNS>(amps, qubits, p, d_ops, batch, st);
+        case 12: return launch_k<float, 12, RUNS>(amps, qubits, p, d_ops, batch, st);
+        case 13: return launch_k<float, 13, RUNS>(amps, qubits, p, d_ops, batch, st);
         default: return cudaErrorInvalidValue;
         }
     }
     switch (p.k) {
-    case 9: return launch_k<double, 9>(amps, qubits, p, d_ops, batch, st);
-    case 10: return launch_k<double, 10>(amps, qubits, p, d_ops, batch, st);
-    case 11: return launch_k<double, 11>(amps, qubits, p, d_ops, batch, st);
-    case 12: return launch_k<double, 12>(amps, qubits, p, d_ops, batch, st);
+    case 9: return launch_k<double, 9, RUNS>(amps, qubits, p, d_ops, batch, st);
+    case 10: return launch_k<double, 10, RUNS>(amps, qubits, p, d_ops, batch, st);
+    case 11: return launch_k<double, 11, RUNS>(amps, qubits, p, d_ops, batch, st);
+    case 12: return launch_k<double, 12, RUNS>(amps, qubits, p, d_ops, batch, st);
     default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_fused(void* amps, int qubits, int precision, const FusedPass& p, const FusedOp* ops,
+                         const FusedOp* d_ops, const FusedBatch* batch, cudaStream_t st) {
+    if (p.k > qubits || p.op_count > kMaxPassOps || p.op_count < 0 || !d_ops) return cudaErrorInvalidValue;
+    if (batch && (batch->states < 1 || batch->states > 65535)) return cudaErrorInvalidValue;
+    bool runs = false;
+    for (int o = p.op_begin + 1; o < p.op_begin + p.op_count; ++o) runs |= (ops[o - 1].flags & ops[o].flags & kOpTurn) != 0;
+    return runs ? launch_fused_t<true>(amps, qubits, precision, p, d_ops, batch, st)
+                : launch_fused_t<false>(amps, qubits, precision, p, d_ops, batch, st);
 }
 
 }  // namespace qm

@@ -245,8 +245,9 @@ struct FusedBatch {
     int32_t slot_count = -1;
     double* hist = nullptr;  // joint-mass partial rows written by a compiled pass with a histogram epilogue
 };
+// ops: the plan's ops; d_ops: their copy in device memory.
 cudaError_t launch_fused(void* amps, int qubits, int precision, const FusedPass& p, const FusedOp* ops,
-                         const FusedBatch* batch, cudaStream_t s);
+                         const FusedOp* d_ops, const FusedBatch* batch, cudaStream_t s);
 
 // Kernel parameters of a fused pass (the interpreter k_fused and the passes compiled for their
 // own op sequence take the same struct; its layout is mirrored in the compiled source).

@@ -2078,7 +2078,7 @@ cudaError_t launch_plan_pass(const Plan& plan, size_t pass, void* amps, const Fu
                                  !plan.jit_aux[pass].empty()
                              ? plan.jit[pass]
                              : nullptr;
-    if (!kernel) return launch_fused(amps, plan.qubits, plan.precision, p, plan.d_ops, batch, st);
+    if (!kernel) return launch_fused(amps, plan.qubits, plan.precision, p, plan.ops.data(), plan.d_ops, batch, st);
     if (batch && (batch->states < 1 || batch->states > 65535)) return cudaErrorInvalidValue;
     FusedLaunch L = fused_launch_params(plan.qubits, p, plan.d_ops, batch);
     const bool fp64 = plan.precision != QM_FP32;
