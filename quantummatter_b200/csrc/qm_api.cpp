@@ -341,7 +341,7 @@ int32_t build_plan(qm_context* ctx, int32_t qubits, int32_t precision, const qm_
         // none there: the interpreter's form of the circuit (27 qubits, complex64,
         // depth 38: 130 ms with the circuit as given, 109 so)
         const bool found = std::any_of(plan.jit.begin(), plan.jit.end(), [](const void* k) { return k != nullptr; });
-        if (!found && (width == 0 || width >= 9)) {
+        if (!found && precision == QM_FP32 && (width == 0 || width >= 9)) {
             Plan again;
             if (!plan_fused(one_shot_gates(list, precision), qubits, precision, width, again, err))
                 return fail(QM_E_ARG, "planner: " + err);

@@ -128,7 +128,7 @@ __device__ __forceinline__ void op_matrix(Cx<T> (&a)[NR], const FusedOp& op, con
     }
 }
 
-// A matrix with a 1 in its first column (kOpRotation): [[1, -t lambda], [t, lambda]], or with B
+// complex64: a matrix with a 1 in its first column (kOpRotation): [[1, -t lambda], [t, lambda]], or with B
 // [[t, -lambda], [1, t lambda]].  The coefficients are t, B and lambda: 8 multiply-adds per pair
 // against 16.
 template <typename T, int M>
@@ -611,29 +611,31 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
         const int words = P.op_count * (int)(sizeof(FusedOp) / sizeof(uint2));
         for (int i = t; i < words; i += blockDim.x) dst[i] = __ldg(src + i);
     }
-    // coefficients in the state's precision, in place, and the matrices that run as rotations
-    __syncthreads();
-    for (int i = t; i < P.op_count; i += blockDim.x) {
-        if (prog[i].code == OP_STAGE || prog[i].code == OP_DIAG_GROUP) continue;
-        double v[8];
+    // complex64: coefficients in the state's precision, in place, and the matrices that run as rotations
+    if constexpr (sizeof(T) == 4) {
+        __syncthreads();
+        for (int i = t; i < P.op_count; i += blockDim.x) {
+            if (prog[i].code == OP_STAGE || prog[i].code == OP_DIAG_GROUP) continue;
+            double v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = prog[i].coef[k];
-        if (prog[i].code == OP_MATRIX && !(prog[i].flags & kOpTable) && prog[i].cmask_local == 0 && v[1] == 0.0 &&
-            v[5] == 0.0 && (v[0] == 1.0 || v[4] == 1.0)) {
-            const bool form_b = v[0] != 1.0;
-            const double tv = form_b ? v[0] : v[4], lr = form_b ? -v[2] : v[6], li = form_b ? -v[3] : v[7];
-            const double er = form_b ? v[6] - tv * lr : v[2] + tv * lr, ei = form_b ? v[7] - tv * li : v[3] + tv * li;
-            if (fabs(er) + fabs(ei) <= 4e-16 * (fabs(lr) + fabs(li))) {
-                prog[i].flags |= kOpRotation;
-                v[0] = tv;
-                v[1] = form_b ? 1.0 : 0.0;
-                v[2] = lr;
-                v[3] = li;
+            for (int k = 0; k < 8; ++k) v[k] = prog[i].coef[k];
+            if (prog[i].code == OP_MATRIX && !(prog[i].flags & kOpTable) && prog[i].cmask_local == 0 && v[1] == 0.0 &&
+                v[5] == 0.0 && (v[0] == 1.0 || v[4] == 1.0)) {
+                const bool form_b = v[0] != 1.0;
+                const double tv = form_b ? v[0] : v[4], lr = form_b ? -v[2] : v[6], li = form_b ? -v[3] : v[7];
+                const double er = form_b ? v[6] - tv * lr : v[2] + tv * lr, ei = form_b ? v[7] - tv * li : v[3] + tv * li;
+                if (fabs(er) + fabs(ei) <= 4e-16 * (fabs(lr) + fabs(li))) {
+                    prog[i].flags |= kOpRotation;
+                    v[0] = tv;
+                    v[1] = form_b ? 1.0 : 0.0;
+                    v[2] = lr;
+                    v[3] = li;
+                }
             }
-        }
-        T* c = reinterpret_cast<T*>(prog[i].coef);
+            T* c = reinterpret_cast<T*>(prog[i].coef);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) c[k] = (T)v[k];
+            for (int k = 0; k < 8; ++k) c[k] = (T)v[k];
+        }
     }
     const int64_t total = (int64_t)P.states << P.cta_shift;
     const uint32_t cta_mask = (1u << P.cta_shift) - 1u;
@@ -721,7 +723,7 @@ __global__ void __launch_bounds__(1 << (K - R), ((sizeof(T) == 8 && K == 12) || 
                 }
             }
             if ((outer & op.cmask_outer) != op.cmask_outer) continue;
-            if (op.flags & kOpRotation) {
+            if (sizeof(T) == 4 && (op.flags & kOpRotation)) {
                 op_rotation_any<T>(a, op.reg, op_coef<T>(op));
                 continue;
             }
