@@ -644,10 +644,12 @@ struct Gen {
     }
 
     // Commuting diagonals as one phase per register.  Members on thread or outer bits fold into one
-    // factor u of the thread; members on register bits become a pair of factors per bit, and the
-    // phases are products of two small tables (four members: 42 complex products against 80 with one
-    // pass over the registers per member).  Table factors on thread bits do not depend on the tile:
-    // with `hoist` they are formed once per state.
+    // factor u of the thread.  Constant members on register bits are multiplied on the host and rounded
+    // once (12 qubits of Clifford and T gates, complex64: 4.0e-7 with products in the kernel).  Those with
+    // coefficients from the table become a pair of factors per bit, and the phases are products of two
+    // small tables (four members: 42 complex products against 80 with one pass over the registers per
+    // member).  Table factors on thread bits do not depend on the tile: with `hoist` they are formed once
+    // per state.
     std::ostringstream* hoist = nullptr;  // code run when a block turns to another state
     std::string hoisted;                  // declarations of what it sets
     void group(int o, const std::vector<FusedOp>& ops, int first, int count) {
@@ -697,6 +699,9 @@ struct Gen {
         }
         staged = staged && !members.empty();
         Factor zero[R], on[R];
+        std::complex<long double> constant[R][2];
+        bool varies[R][2] = {};
+        for (auto& c : constant) c[0] = c[1] = 1.0L;
         for (int k = 0; k < count; ++k) {
             const FusedOp& m = ops[(size_t)(first + k)];
             const int om = o + 1 + k;
@@ -707,6 +712,18 @@ struct Gen {
             const int M = m.local >= 0 ? reg_of_local(m.local) : -1;
             if (M >= 0) {
                 if (staged) continue;
+                if (!(m.flags & kOpTable)) {
+                    if (aux.size() + 2 * NR > kMaxAuxValues) {
+                        diag(om, m);
+                        continue;
+                    }
+                    for (int v = 0; v < 2; ++v) {
+                        if (m.flags & (1 << v)) continue;  // exactly 1
+                        constant[M][v] *= std::complex<long double>(m.coef[6 * v], m.coef[6 * v + 1]);
+                        varies[M][v] = true;
+                    }
+                    continue;
+                }
                 const std::string c = coef_ptr(om, m), n = std::to_string(uid++);
                 os << "const " << T << " zr" << n << " = (" << T << ")" << c << "[0], zi" << n << " = (" << T << ")" << c
                    << "[1], or" << n << " = (" << T << ")" << c << "[6], oi" << n << " = (" << T << ")" << c << "[7];\n";
@@ -718,6 +735,23 @@ struct Gen {
             const int n = open_conditions(m.cmask_outer, 0);
             fold_member(os, m, om, "ur", "ui");
             close(n);
+        }
+        std::vector<int> constant_slot(1 << R, -1);  // one constant per distinct phase
+        for (int i = 0; i < NR; ++i) {
+            std::complex<long double> p = 1.0L;
+            int same = 0;  // the register with this phase: only bits with a member count
+            bool one = true;
+            for (int m = 0; m < R; ++m) {
+                const int v = (i >> m) & 1;
+                if (!varies[m][0] && !varies[m][1]) continue;
+                same |= v << m;
+                if (!varies[m][v]) continue;
+                p *= constant[m][v];
+                one = false;
+            }
+            if (one) continue;
+            if (constant_slot[same] < 0) constant_slot[same] = slot2(cplx((double)p.real(), (double)p.imag()));
+            cmul_reg(i, av(constant_slot[same]).c_str(), av(constant_slot[same] + 1).c_str());
         }
         std::vector<int> bits;
         for (int m = 0; m < R; ++m)
