@@ -100,8 +100,10 @@ typedef struct qm_gate {
 typedef struct qm_options {
     int32_t device_index;
     int32_t enable_profiling;       /* fills qm_profile in the *_profiled calls */
-    int64_t device_budget_bytes;    /* maximum bytes of device states held by the context */
-    int64_t staging_budget_bytes;   /* maximum pinned host staging bytes */
+    int64_t device_budget_bytes;    /* maximum bytes of device states held by the context; up to 128 MiB
+                                       of a batch call's memory stay with it, within this budget */
+    int64_t staging_budget_bytes;   /* maximum pinned host staging bytes; up to 32 MiB of a batch call's
+                                       transfer buffers stay, within this budget */
     int32_t fusion_width;           /* 0 = planner default (fused blocks of 12 qubits); 1 = one launch
                                        per gate; 2..6 = dense fused gates of at most that many qubits,
                                        one sweep of the state each; 9..14 = fused blocks of that many

@@ -40,19 +40,58 @@ int32_t cuda_fail(cudaError_t err, const char* what) {
 
 using namespace qm;
 
+namespace {
+
+std::mutex g_pools_mu;
+std::vector<cudaMemPool_t> g_pools;  // of every context
+
+// Runs `allocate` again without what the contexts' pools keep idle when the device has no memory left.
+template <typename Allocate>
+cudaError_t retried(qm_context* ctx, Allocate allocate) {
+    cudaError_t e = allocate();
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);  // frees queued on it
+    {
+        std::lock_guard<std::mutex> lock(g_pools_mu);
+        if (g_pools.empty()) return e;
+        for (cudaMemPool_t pool : g_pools) cudaMemPoolTrimTo(pool, 0);
+    }
+    return allocate();
+}
+
+}  // namespace
+
+cudaError_t device_alloc(qm_context* ctx, void** out, size_t bytes) {
+    return retried(ctx, [&] { return cudaMalloc(out, bytes); });
+}
+
 cudaError_t pool_alloc(qm_context* ctx, void** out, size_t bytes) {
-    if (bytes > kPoolKeep) return cudaMalloc(out, bytes);
+    if (bytes > kPoolKeep) return device_alloc(ctx, out, bytes);
     if (!ctx->pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = ctx->device;
         cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
-        uint64_t keep = kPoolKeep;
-        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
         if (e != cudaSuccess) return e;
+        uint64_t keep = std::min<uint64_t>(kPoolKeep, (uint64_t)ctx->device_budget);
+        e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> lock(g_pools_mu);
+        g_pools.push_back(ctx->pool);
     }
-    return cudaMallocFromPoolAsync(out, bytes, ctx->pool, ctx->stream);
+    return retried(ctx, [&] { return cudaMallocFromPoolAsync(out, bytes, ctx->pool, ctx->stream); });
+}
+
+void make_room(qm_context* ctx, int64_t bytes) {
+    if (!ctx->pool) return;
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return;
+    const uint64_t room = (uint64_t)std::max<int64_t>(0, ctx->device_budget - ctx->device_in_use - bytes);
+    if (reserved - used > room) cudaMemPoolTrimTo(ctx->pool, used + room);
 }
 
 void pool_free(qm_context* ctx, void* pointer, size_t bytes) {
@@ -76,7 +115,7 @@ int32_t ensure_scratch(qm_context* ctx, size_t bytes) {
         ctx->scratch_bytes = 0;
     }
     size_t sz = std::max<size_t>(bytes, 1 << 20);
-    QM_CUDA(cudaMalloc(&ctx->scratch, sz));
+    QM_CUDA(device_alloc(ctx, &ctx->scratch, sz));
     ctx->scratch_bytes = sz;
     return QM_OK;
 }
@@ -241,18 +280,19 @@ int32_t validate_prepared_gates(const qm_gate* gates, int32_t count, int32_t qub
     return validate_gates(gates, count, qubits);
 }
 
-int32_t plan_upload(Plan& plan, cudaStream_t stream, void** buffer, size_t* buffer_bytes) {
+int32_t plan_upload(Plan& plan, qm_context* ctx, void** buffer, size_t* buffer_bytes) {
+    const cudaStream_t stream = ctx->stream;
     if (!plan.dense.empty() && !plan.d_status) {
-        QM_CUDA(cudaMalloc(&plan.d_status, sizeof(int32_t)));
+        QM_CUDA(device_alloc(ctx, reinterpret_cast<void**>(&plan.d_status), sizeof(int32_t)));
         QM_CUDA(cudaMemsetAsync(plan.d_status, 0, sizeof(int32_t), stream));
         if (!plan.dense_matrices.empty()) {
             const size_t mbytes = plan.dense_matrices.size() * sizeof(double);
-            QM_CUDA(cudaMalloc(&plan.d_dense, mbytes));
+            QM_CUDA(device_alloc(ctx, reinterpret_cast<void**>(&plan.d_dense), mbytes));
             QM_CUDA(cudaMemcpyAsync(plan.d_dense, plan.dense_matrices.data(), mbytes, cudaMemcpyHostToDevice, stream));
         }
         if (!plan.dense_tc.empty()) {
             const size_t ibytes = plan.dense_tc.size() * sizeof(float);
-            QM_CUDA(cudaMalloc(&plan.d_dense_tc, ibytes));
+            QM_CUDA(device_alloc(ctx, reinterpret_cast<void**>(&plan.d_dense_tc), ibytes));
             QM_CUDA(cudaMemcpyAsync(plan.d_dense_tc, plan.dense_tc.data(), ibytes, cudaMemcpyHostToDevice, stream));
         }
     }
@@ -266,13 +306,13 @@ int32_t plan_upload(Plan& plan, cudaStream_t stream, void** buffer, size_t* buff
             }
             *buffer = nullptr;
             *buffer_bytes = 0;
-            QM_CUDA(cudaMalloc(buffer, bytes * 2));
+            QM_CUDA(device_alloc(ctx, buffer, bytes * 2));
             *buffer_bytes = bytes * 2;
         }
         plan.d_ops = static_cast<FusedOp*>(*buffer);
         plan.borrowed = true;
     } else {
-        QM_CUDA(cudaMalloc(&plan.d_ops, bytes));
+        QM_CUDA(device_alloc(ctx, reinterpret_cast<void**>(&plan.d_ops), bytes));
     }
     QM_CUDA(cudaMemcpyAsync(plan.d_ops, plan.ops.data(), bytes, cudaMemcpyHostToDevice, stream));
     return QM_OK;
@@ -348,8 +388,8 @@ int32_t build_plan(qm_context* ctx, int32_t qubits, int32_t precision, const qm_
             plan = std::move(again);
         }
     }
-    if (transient) return plan_upload(plan, ctx->stream, &ctx->program, &ctx->program_bytes);
-    return plan_upload(plan, ctx->stream);
+    if (transient) return plan_upload(plan, ctx, &ctx->program, &ctx->program_bytes);
+    return plan_upload(plan, ctx);
 }
 
 void free_plan(Plan& plan) { plan_release(plan); }
@@ -512,7 +552,11 @@ extern "C" int32_t qm_context_destroy(qm_context* ctx) {
         if (ctx->staging) cudaFree(ctx->staging);
         if (ctx->program) cudaFree(ctx->program);
         if (ctx->pinned) cudaFreeHost(ctx->pinned);
-        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+        if (ctx->pool) {
+            std::lock_guard<std::mutex> pools(g_pools_mu);
+            g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), ctx->pool), g_pools.end());
+            cudaMemPoolDestroy(ctx->pool);
+        }
         release_bounce(ctx);
         if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
         if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
@@ -562,7 +606,8 @@ int32_t device_buffer(qm_context* ctx, size_t bytes, void** out) {
             ctx->staging = nullptr;
             ctx->staging_bytes = 0;
         }
-        QM_CUDA(cudaMalloc(&ctx->staging, bytes));
+        make_room(ctx, (int64_t)bytes);
+        QM_CUDA(device_alloc(ctx, &ctx->staging, bytes));
         ctx->staging_bytes = bytes;
     }
     *out = ctx->staging;
@@ -767,14 +812,9 @@ extern "C" int32_t qm_state_create(qm_context* ctx, int32_t qubits, int32_t prec
     st->qubits = qubits;
     st->precision = precision;
     st->bytes = bytes;
-    cudaError_t e = cudaMalloc(&st->amps, (size_t)bytes);
-    if (e == cudaErrorMemoryAllocation && ctx->pool) {  // what the pool keeps may be what is missing
-        cudaGetLastError();
-        cudaMemPoolTrimTo(ctx->pool, 0);
-        e = cudaMalloc(&st->amps, (size_t)bytes);
-    }
-    QM_CUDA(e);
-    e = launch_reset(st->amps, qubits, precision, ctx->stream);
+    make_room(ctx, bytes);
+    QM_CUDA(device_alloc(ctx, &st->amps, (size_t)bytes));
+    cudaError_t e = launch_reset(st->amps, qubits, precision, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(st->amps);
@@ -1036,7 +1076,8 @@ extern "C" int32_t qm_plan_autotune(qm_context* ctx, int32_t qubits, int32_t pre
         if ((int64_t)bytes + ctx->device_in_use > ctx->device_budget)
             return fail(QM_E_BUDGET, "autotuning needs a scratch state within the device budget");
         void* scratch = nullptr;
-        QM_CUDA(cudaMalloc(&scratch, bytes));
+        make_room(ctx, (int64_t)bytes);
+        QM_CUDA(device_alloc(ctx, &scratch, bytes));
         double best_s = 0;
         for (int32_t w : widths) {
             Plan plan;

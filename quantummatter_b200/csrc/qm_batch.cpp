@@ -215,6 +215,7 @@ extern "C" int32_t qm_batch_create(qm_context* ctx, int32_t qubits, int32_t prec
     b->precision = precision;
     b->capacity = capacity;
     b->state_bytes = state_bytes;
+    make_room(ctx, bytes);
     QM_CUDA(pool_alloc(ctx, &b->amps, (size_t)bytes));
     cudaError_t e = launch_reset_batched(b->amps, qubits, precision, capacity, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -239,6 +240,7 @@ extern "C" int32_t qm_batch_destroy(qm_batch* b) {
         pool_free(b->ctx, b->out, b->out_bytes);
         cudaStreamSynchronize(b->ctx->stream);  // beyond kPoolKeep the pool gives memory back here
         b->ctx->device_in_use -= b->state_bytes * b->capacity;
+        make_room(b->ctx, 0);
     }
     delete b;
     return QM_OK;
@@ -269,7 +271,7 @@ extern "C" int32_t qm_batch_state(qm_batch* b, int32_t index, double* amplitudes
         else QM_CUDA(cudaMemcpyAsync(amplitudes, base, (size_t)b->state_bytes, cudaMemcpyDeviceToHost, ctx->stream));
     } else {
         double* tmp = nullptr;
-        QM_CUDA(cudaMalloc(&tmp, (size_t)(16 * length)));
+        QM_CUDA(device_alloc(ctx, reinterpret_cast<void**>(&tmp), (size_t)(16 * length)));
         cudaError_t e;
         if (upload) {
             e = cudaMemcpyAsync(tmp, amplitudes, (size_t)(16 * length), cudaMemcpyHostToDevice, ctx->stream);
@@ -313,7 +315,7 @@ extern "C" int32_t qm_batch_execute(qm_batch* b, int32_t states, const qm_gate* 
         Plan& p;
         ~Release() { plan_release(p); }
     } release{plan};
-    rc = plan_upload(plan, ctx->stream);
+    rc = plan_upload(plan, ctx);
     if (rc) return rc;
     const size_t tbytes = sizeof(double) * (size_t)states * slot_count * 8;
     if (tbytes) {
@@ -738,7 +740,7 @@ int32_t run_problems(qm_context* ctx, std::vector<std::unique_ptr<VqeProblem>>& 
     struct PinnedGuard {  // a large block is not kept
         qm_context* ctx;
         ~PinnedGuard() {
-            if (ctx->pinned_bytes <= kPinnedKeep) return;
+            if (ctx->pinned_bytes <= std::min<uint64_t>(kPinnedKeep, (uint64_t)ctx->staging_budget)) return;
             cudaStreamSynchronize(ctx->stream);
             cudaFreeHost(ctx->pinned);
             ctx->pinned = nullptr;

@@ -185,7 +185,7 @@ struct Plan {
 // Copies the plan's program to the device (stream-ordered) / frees it.  With `buffer`, the
 // program goes into that growable device buffer instead of a new allocation (transient plans
 // of one-shot executions).
-int32_t plan_upload(Plan& plan, cudaStream_t stream, void** buffer = nullptr, size_t* buffer_bytes = nullptr);
+int32_t plan_upload(Plan& plan, qm_context* ctx, void** buffer = nullptr, size_t* buffer_bytes = nullptr);
 void plan_release(Plan& plan);
 
 // Builds the fused schedule (qm_planner.cpp).  Returns false with a message on error.
@@ -513,9 +513,14 @@ struct qm_context {
 // Device memory of a batch call on the context's stream, the same `bytes` to free it; callers hold the
 // context's lock.  Up to kPoolKeep bytes come from the context's pool; larger ones are plain
 // allocations (1.6 GB through the pool is mapped anew on each call: 10 ms more per trajectory run).
+// What a pool keeps idle stays within the context's device budget beside its states (make_room: and
+// beside `bytes` more of them), and goes back to the device when any allocation finds it full.  Page-locked
+// memory is kept within the staging budget.
 constexpr uint64_t kPoolKeep = 128ull << 20;
 constexpr size_t kPinnedKeep = 32u << 20;
+cudaError_t device_alloc(qm_context* ctx, void** out, size_t bytes);  // cudaMalloc
 cudaError_t pool_alloc(qm_context* ctx, void** out, size_t bytes);
+void make_room(qm_context* ctx, int64_t bytes);
 void pool_free(qm_context* ctx, void* pointer, size_t bytes);
 // Whole-state copies with a caller's host buffer on the context's stream (qm_transfer.cpp):
 // host_to_device returns once the host buffer has been read (the device copy may still be in

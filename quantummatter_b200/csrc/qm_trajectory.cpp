@@ -272,6 +272,7 @@ struct Buffers {
         for (auto& p : ptrs) pool_free(ctx, p.first, p.second);
         cudaStreamSynchronize(stream);
         ctx->device_in_use -= accounted;
+        make_room(ctx, 0);
     }
     template <typename T>
     int32_t get(T*& out, size_t bytes) {
@@ -346,6 +347,7 @@ extern "C" int32_t qm_trajectories_run(qm_context* ctx, int32_t qubits, int32_t 
     Buffers buf(ctx);
     buf.accounted = B * per_state((int)B) + fixed;
     ctx->device_in_use += buf.accounted;
+    make_room(ctx, 0);
     void* amps = nullptr;
     double *table = nullptr, *partials = nullptr, *d_draws = nullptr, *tpart = nullptr, *tout = nullptr;
     double *d_masses = nullptr, *mean = nullptr, *m2 = nullptr;
