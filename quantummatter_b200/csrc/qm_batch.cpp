@@ -459,7 +459,6 @@ struct VqeProblem {
     VqeProblem(const VqeProblem&) = delete;
     VqeProblem& operator=(const VqeProblem&) = delete;
     ~VqeProblem() {
-        if (own_stream && stream) cudaStreamSynchronize(stream);  // work of a wave that failed to join
         if (program) {
             std::lock_guard<std::recursive_mutex> lock(owner->mu);
             pool_free(owner, program, program_bytes);
@@ -737,16 +736,21 @@ int32_t run_problems(qm_context* ctx, std::vector<std::unique_ptr<VqeProblem>>& 
         QM_CUDA(cudaMallocHost(&ctx->pinned, pinned));
         ctx->pinned_bytes = pinned;
     }
-    struct PinnedGuard {  // a large block is not kept
+    // The context's lock ends with this function: whatever way it is left, no problem's copies may still
+    // use the block then.  A large one is not kept.
+    struct PinnedGuard {
         qm_context* ctx;
+        std::vector<std::unique_ptr<VqeProblem>>& problems;
         ~PinnedGuard() {
-            if (ctx->pinned_bytes <= std::min<uint64_t>(kPinnedKeep, (uint64_t)ctx->staging_budget)) return;
+            for (auto& p : problems)
+                if (p->own_stream) cudaStreamSynchronize(p->stream);
             cudaStreamSynchronize(ctx->stream);
+            if (ctx->pinned_bytes <= std::min<uint64_t>(kPinnedKeep, (uint64_t)ctx->staging_budget)) return;
             cudaFreeHost(ctx->pinned);
             ctx->pinned = nullptr;
             ctx->pinned_bytes = 0;
         }
-    } pinned_guard{ctx};
+    } pinned_guard{ctx, problems};
     double* host = static_cast<double*>(ctx->pinned);
     for (auto& p : problems) host = p->host_buffers(host);
     const bool multi = problems.size() > 1;
