@@ -378,10 +378,15 @@ int32_t build_plan(qm_context* ctx, int32_t qubits, int32_t precision, const qm_
     // so those run the interpreter.
     if (transient && qubits >= 26) {
         jit_lookup(plan);
-        // none there: the interpreter's form of the circuit (27 qubits, complex64,
-        // depth 38: 130 ms with the circuit as given, 109 so)
-        const bool found = std::any_of(plan.jit.begin(), plan.jit.end(), [](const void* k) { return k != nullptr; });
-        if (!found && precision == QM_FP32 && (width == 0 || width >= 9)) {
+        // few there: the interpreter's form of the circuit (27 qubits, complex64, depth 38: 130 ms with
+        // the circuit as given, 109 so).  A compiled pass takes a fifth of an interpreted one, so a
+        // quarter of the ops in compiled passes makes up for the others as given.
+        int64_t ops = 0, compiled = 0;
+        for (size_t i = 0; i < plan.passes.size(); ++i) {
+            ops += plan.passes[i].op_count;
+            if (plan.jit[i]) compiled += plan.passes[i].op_count;
+        }
+        if (4 * compiled < ops && precision == QM_FP32 && (width == 0 || width >= 9)) {
             Plan again;
             if (!plan_fused(one_shot_gates(list, precision), qubits, precision, width, again, err))
                 return fail(QM_E_ARG, "planner: " + err);
