@@ -248,10 +248,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pauli_sum(const typename Vec2<T
                 }
             }
             KSum w{((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])), 0.0};
-            if (L.tiles > gridDim.x)
-                for (int d = 16; d > 0; d >>= 1) w.merge(shfl_down_ksum(w, d));
-            else  // a single tile: eleven plain additions (a small state's one warp takes 22 such sums)
-                w.s = warp_total(w.s);
+            for (int d = 16; d > 0; d >>= 1) w.merge(shfl_down_ksum(w, d));
             if (lane == 0) totals[i].merge(w);
         }
     };
