@@ -1306,9 +1306,9 @@ int32_t validate_terms(const qm_pauli_term* terms, int32_t count, int qubits) {
     return QM_OK;
 }
 
-// Raw sums of the terms and the mass of a state of at least 9 qubits through the tiled kernel, whose
-// tiles hold flip masks of any width up to a tile; false when a mask spans more.
-bool tiled_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, int32_t* rc) {
+// Raw sums of the terms and (not null) the mass of a state of at least 9 qubits through the tiled kernel,
+// whose tiles hold flip masks of any width up to a tile; false when a mask spans more.
+bool tiled_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, double* mass, int32_t* rc) {
     qm_context* ctx = st->ctx;
     TilePlan tp;
     std::string err;
@@ -1330,10 +1330,37 @@ bool tiled_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, 
                                 ctx->stream));
         QM_CUDA(cudaStreamSynchronize(ctx->stream));
         for (int32_t i = 0; i < count; ++i) raw[i] = ctx->host_scratch[i];
+        if (mass) *mass = ctx->host_scratch[tp.mass_column];
         return QM_OK;
     };
     *rc = run();
     return true;
+}
+
+// Diagonal terms and the mass through the tiled kernel, which takes up to kTileMaxTerms of them from one
+// transform per tile; a phase is a sign here, or makes the term zero.  The list goes through in one piece,
+// with one wait, while its table of sums per tile and pass stays below 32 MiB, and else a pass at a time:
+// 1000 Z strings, complex128: 110 us against 198 in four pieces at 16 qubits, 472 against 421 at 22.
+int32_t tiled_diagonals(qm_state* st, const qm_pauli_term* terms, size_t count, double* raw, double* mass) {
+    const size_t tiles = (size_t)1 << (st->qubits - tile_block_qubits(st->qubits, st->precision));
+    const size_t passes = (count + kTileMaxTerms - 1) / kTileMaxTerms;
+    const size_t piece = sizeof(double) * tiles * passes * count <= (32u << 20) ? count : (size_t)kTileMaxTerms;
+    std::vector<qm_pauli_term> some;
+    for (size_t at = 0; at == 0 || at < count; at += piece) {
+        const size_t n = std::min(count - at, piece);
+        const qm_pauli_term* list = terms + at;
+        if (std::any_of(list, list + n, [](const qm_pauli_term& t) { return (t.y_count & 3) != 0; })) {
+            some.assign(list, list + n);
+            for (qm_pauli_term& t : some) t.y_count = 0;
+            list = some.data();
+        }
+        int32_t rc = QM_OK;
+        tiled_expectation(st, list, (int32_t)n, raw + at, at == 0 ? mass : nullptr, &rc);
+        if (rc) return rc;
+        for (size_t i = at; i < at + n; ++i)
+            if (int phase = terms[i].y_count & 3) raw[i] = (phase & 1) ? 0.0 : -raw[i];
+    }
+    return QM_OK;
 }
 
 // The same with the mass, one pass per distinct flip mask: any state and any mask.
@@ -1360,13 +1387,15 @@ int32_t grouped_expectation(qm_state* st, const qm_pauli_term* terms, int32_t co
 }
 
 // Raw term sums and mass into host arrays (raw[count], *mass).  States of 9 or more qubits take the
-// whole term list in a few reads of the state (qm_pauli_sum.cu), but for terms that flip more than
-// four qubits, which share the tiled kernel's passes; smaller states run one pass per flip mask.
+// whole term list in a few reads of the state (qm_pauli_sum.cu), but for what its plan leaves out: terms
+// that flip more than four qubits and long lists of diagonal ones (all terms, if there are no others),
+// which go through the tiled kernel.  Smaller states run one pass per flip mask.
 int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t count, double* raw, double* mass) {
     if (st->qubits < 9) return grouped_expectation(st, terms, count, raw, mass);
     qm_context* ctx = st->ctx;
     PauliSumPlan plan;
     plan_pauli_sum(st->qubits, st->precision, terms, count, ctx->sm_count, plan);
+    if (plan.passes == 0) return tiled_diagonals(st, terms, (size_t)count, raw, mass);
     const size_t program = pauli_sum_inline(plan) ? 0 : (plan.program.size() + 255) & ~size_t(255);
     const size_t masses = (size_t)plan.parts * plan.tiles, cells = (size_t)plan.grid * plan.columns;
     const size_t folds = pauli_sum_folds(plan);
@@ -1390,16 +1419,18 @@ int32_t device_expectation(qm_state* st, const qm_pauli_term* terms, int32_t cou
     QM_CUDA(cudaStreamSynchronize(ctx->stream));
     for (int32_t i = 0; i < count; ++i) raw[i] = host[i];
     *mass = host[count];
-    if (plan.wide.empty()) return QM_OK;
-    std::vector<qm_pauli_term> wide;
-    for (int i : plan.wide) wide.push_back(terms[i]);
-    std::vector<double> sums(wide.size());
-    if (!tiled_expectation(st, wide.data(), (int32_t)wide.size(), sums.data(), &rc)) {
+    std::vector<qm_pauli_term> wide, diagonal;
+    for (int i : plan.wide) (terms[i].flip_mask ? wide : diagonal).push_back(terms[i]);
+    std::vector<double> sums(plan.wide.size()), diagonal_sums(diagonal.size());
+    if (!wide.empty() && !tiled_expectation(st, wide.data(), (int32_t)wide.size(), sums.data(), nullptr, &rc)) {
         double again = 0;
         rc = grouped_expectation(st, wide.data(), (int32_t)wide.size(), sums.data(), &again);
     }
-    for (size_t i = 0; rc == QM_OK && i < wide.size(); ++i) raw[plan.wide[i]] = sums[i];
-    return rc;
+    if (rc == QM_OK && !diagonal.empty()) rc = tiled_diagonals(st, diagonal.data(), diagonal.size(), diagonal_sums.data(), nullptr);
+    if (rc) return rc;
+    size_t w = 0, d = 0;
+    for (int i : plan.wide) raw[i] = terms[i].flip_mask ? sums[w++] : diagonal_sums[d++];
+    return QM_OK;
 }
 
 }  // namespace

@@ -335,8 +335,9 @@ cudaError_t launch_measure(void* amps, int qubits, int precision, uint64_t mask,
 
 // ---------------------------------------------------------------- Pauli sums of one state (qm_pauli_sum.cu)
 // The passes of a term list over a state of at least 9 qubits: `program` is their device form, `wide`
-// the terms left out (they flip more than four qubits).  Terms that are zero for every state keep a
-// zero column.
+// the terms left out (they flip more than four qubits, or are many diagonal ones).  No passes: the list
+// is diagonal and belongs to the tiled kernel, with the mass.  Terms that are zero for every state keep
+// a zero column.
 struct PauliSumPlan {
     int qubits = 0, k = 0, passes = 0, diagonal_passes = 0, parts = 0, locals = 0, outers = 0, max_entries = 0, columns = 0;
     uint32_t tiles = 0, grid = 0;

@@ -17,7 +17,8 @@
 // - Diagonal terms.  Signs on tile qubits only: every thread sums its 16 probabilities over its
 //   tiles, and one Walsh-Hadamard transform per block at the end gives every such term.  Signs on
 //   outer qubits too: the tile's signed mass for each distinct tile part is written per tile, and
-//   k_outer_terms sums those with the signs of the tile index.
+//   k_outer_terms sums those with the signs of the tile index.  Many of them, and lists of nothing else,
+//   are left to the tiled kernel (plan_pauli_sum has the rule).
 // Products and sums are FP64 for both precisions (complex64 amplitudes widen when they are loaded).
 // No value goes through more plain additions than in a reduction of every tile by itself (19 for a
 // flip's pairs: 7 in a thread, 5 in a warp, 7 over warps; 12 in a tile's transform).  A running sum is
@@ -446,6 +447,12 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
     plan.tiles = 1u << (qubits - k);
     plan.grid = std::min<uint32_t>(plan.tiles, 2u * (uint32_t)std::max(1, sm_count));
 
+    uint32_t flips = 0, signs = 0;
+    for (int i = 0; i < count; ++i) {
+        flips |= terms[i].flip_mask;
+        signs |= terms[i].sign_mask;
+    }
+    if (flips == 0 && (signs & ~first_tile) && plan.tiles <= 1024) return;  // the rule stands below
     std::vector<SumPass> passes;
     std::vector<SumStage> stages;
     std::vector<SumEntry> entries;
@@ -455,6 +462,7 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
 
     std::vector<int> pending;
     std::vector<uint32_t> part_masks;
+    std::vector<int32_t> part_of((size_t)1 << k, -1);  // of a tile part
     locals.push_back(SumLocal{1.0, 0u, count});  // the Born mass
     for (int i = 0; i < count; ++i) {
         const qm_pauli_term& t = terms[i];
@@ -470,16 +478,32 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
                 locals.push_back(SumLocal{unit(negate), local, i});
                 continue;
             }
-            size_t p = 0;
-            while (p < part_masks.size() && part_masks[p] != local) ++p;
-            if (p == part_masks.size()) part_masks.push_back(local);
-            outers.push_back(SumOuter{unit(negate), outer >> k, (int32_t)p, i, 0});
+            if (part_of[local] < 0) {
+                part_of[local] = (int32_t)part_masks.size();
+                part_masks.push_back(local);
+            }
+            outers.push_back(SumOuter{unit(negate), outer >> k, part_of[local], i, 0});
             continue;
         }
         const bool cancels = ((__builtin_popcount(t.flip_mask & t.sign_mask) ^ phase) & 1) != 0;  // pair by pair: zero
         if (cancels) plan.zeros = true;
         else if (__builtin_popcount(t.flip_mask) > 4) plan.wide.push_back(i);
         else pending.push_back(i);
+    }
+    // Diagonal terms with outer signs cost a warp reduction per distinct tile part and tile here, and a read
+    // of the state per kMaxParts of them; the tiled kernel (qm_expect.cu) takes 256 terms from one
+    // transform per tile, at a row of sums per tile and, beside flips, a read and a wait of its own.
+    // It takes diagonal lists of states of up to 22 qubits, longer ones of larger states and long ones
+    // beside flips.  Random Z strings alone (complex128, sums here / tiled): 16 of them 37 / 34 us at 18
+    // qubits, 73 / 58 at 22, 97 / 85 at 23, 148 / 139 at 24, 8 of them 111 / 135 at 24, 256 of them 205 / 54
+    // at 18 and 1736 / 301 at 24.  Beside as many flips: 16 of them 65 / 93 us at 20 qubits, 410 / 465 at
+    // 24; 32 of them 84 / 95 and 590 / 519; 128 of them 68 / 102 at 16, 167 / 114 at 18 and 217 / 159 at 20.
+    const int distinct = (int)part_masks.size();
+    if (flips == 0 && distinct > kMaxParts) return;
+    if (plan.tiles >= 64 && distinct > 2 * kMaxParts) {
+        for (const SumOuter& o : outers) plan.wide.push_back(o.column);
+        outers.clear();
+        part_masks.clear();
     }
     // neighbouring flips side by side, so that a tile and a stage take as many as they can
     std::stable_sort(pending.begin(), pending.end(), [&](int x, int y) {
@@ -498,12 +522,17 @@ void plan_pauli_sum(int qubits, int precision, const qm_pauli_term* terms, int c
         int pairs = 0;
         bool half = false;
         uint64_t last_kind = 0;
-        for (int i : pending) {
+        for (size_t j = 0; j < pending.size(); ++j) {
+            const int i = pending[j];
             const uint32_t nq = Q | terms[i].flip_mask;
             // a new pair of sums, or the second half of the last one (terms of one flip and part are neighbours)
             const uint64_t kind = ((uint64_t)terms[i].flip_mask << 1) | (uint64_t)(terms[i].y_count & 1);
             const bool opens = !half || kind != last_kind;
-            if (pairs + (opens ? 1 : 0) <= kEntries && __builtin_popcount(nq) <= k) {
+            if (pairs == kEntries && opens) {  // full: so is the pass for all terms behind
+                rest.insert(rest.end(), pending.begin() + (std::ptrdiff_t)j, pending.end());
+                break;
+            }
+            if (__builtin_popcount(nq) <= k) {
                 Q = nq;
                 mine.push_back(i);
                 pairs += opens ? 1 : 0;
