@@ -46,3 +46,24 @@ def test_dense_gates_match_the_oracle(gpu_context, m, n, precision, tol):
             st.Upload(psi)
             st.Evolve(c, fusion_width=m)
             assert np.max(np.abs(st.Download() - want)) <= tol, qubits
+
+
+@pytest.mark.parametrize("qubits", [list(range(6)), list(range(17, 23)), [0, 4, 9, 13, 18, 22], [0, 1, 2, 20, 21, 22],
+                                    [7, 8, 9, 10, 11, 12]], ids=lambda q: "-".join(map(str, q)))
+def test_full_tiles_match_a_launch_per_gate(gpu_context, qubits):
+    """Six qubits of 23, complex128: tiles of 4096 amplitudes, fourteen per block in a ring of three.
+    Amplitudes of 3.5e-4; 1e-17 is some hundred roundings of one."""
+    n, rng = 23, np.random.default_rng(qubits[-1])
+    c = QuantumCircuit(n)
+    for _ in range(2):
+        for q in qubits:
+            c.Ry(q, float(rng.uniform(0, 6.28))).Rz(q, float(rng.uniform(0, 6.28)))
+        for a, b in zip(qubits, qubits[1:]):
+            c.CNot(a, b)
+    psi, got = random_state(n, qubits[0]), {}
+    for width in (6, 1):
+        with DeviceState(gpu_context, n, FP64) as st:
+            st.Upload(psi)
+            st.Evolve(c, fusion_width=width)
+            got[width] = st.Download()
+    assert np.max(np.abs(got[6] - got[1])) <= 1e-17
