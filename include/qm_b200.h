@@ -400,7 +400,8 @@ typedef struct qm_vqe_stats {
  * parameter vectors at once: parameters[vector][parameter_count] -> energies[vector] and, when
  * with_gradient != 0, gradients[vector][parameter_count] by the occurrence-wise +-pi/2
  * parameter-shift rule with termwise differencing and Neumaier accumulation.  Every base and
- * shifted circuit runs as a state of device batches (waves sized by the device budget).
+ * shifted circuit runs as a state of device batches: waves of 64 MiB of states (the second-level
+ * cache holds them), more where that leaves the device short of work, within the device budget.
  * stats may be NULL. */
 int32_t qm_vqe_evaluate(qm_context* context, int32_t qubits, int32_t precision, const qm_template_op* operations,
                         int32_t operation_count, int32_t parameter_count, const qm_pauli_term* terms,
@@ -418,8 +419,8 @@ int32_t qm_vqe_evaluate_coefficients(qm_context* context, int32_t qubits, int32_
 /* Several evaluations of different sizes at once (the batched form of VariationalEnergyEvaluator
  * for a mix of registers, e.g. 16-, 18-, 20- and 22-qubit ansatzes).  Each problem is what one
  * qm_vqe_evaluate / qm_vqe_evaluate_coefficients call takes (coefficients NULL: the terms' own).
- * The device budget is shared in proportion to each problem's state bytes; every round runs each
- * problem's next wave on its own stream, forked from and joined to the context's stream, so the
+ * The device budget and a wave's 64 MiB are shared in proportion to each problem's state bytes times
+ * its circuits; every round runs each problem's next wave on its own stream, forked from and joined to the context's stream, so the
  * sizes overlap on the device, and rounds in which every problem runs a full wave replay one
  * captured CUDA graph (one launch for all sizes).  Results equal the separate calls'. */
 typedef struct qm_vqe_problem {

@@ -19,7 +19,7 @@
 //     where its index bits form at most five runs, else by 16-byte cp.async of four producer warps,
 //     which also write it back (27 qubits, gate on 0, 4, 9, 13, 18 and 24: 33 ms with a bulk copy per
 //     run of two amplitudes, 0.54 ms so; 0.49 ms as boxes on neighbouring qubits);
-//   - all 256 threads split the tile into B_hi / B_lo in the canonical K-major layout of the
+//   - 16 warps split the tile into B_hi / B_lo in the canonical K-major layout of the
 //     MMA (two B buffers, so tile i converts while tile i-1's MMAs run);
 //   - one thread issues the 24 MMAs of the tile (8 K-steps x 3 products, M = 128, N = 64, K = 8)
 //     into one of two TMEM accumulators and commits them to an mbarrier;
@@ -587,8 +587,8 @@ bool dense_tc_supported(int qubits, int precision, const DenseOp& op) {
 }
 
 // On unless QM_DENSE_TC=0; read at every plan, so a process can plan with and without the tensor
-// cores.  Measured on the 30-qubit brick (complex64): dense fused gates of <= 5 qubits 1237 against
-// 1693 ms per step, of <= 6 qubits 1760 against 2601 ms, with the largest amplitude error against
+// cores.  Measured on the 30-qubit brick (complex64): dense fused gates of <= 5 qubits 698 against
+// 1693 ms per step, of <= 6 qubits 633 against 2601 ms, with the largest amplitude error against
 // complex128 1.4e-8 against 3e-10 (3xTF32 keeps about 21 significant bits per product).
 bool dense_tc_enabled() {
     const char* e = std::getenv("QM_DENSE_TC");

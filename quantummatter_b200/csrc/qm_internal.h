@@ -222,7 +222,7 @@ cudaError_t launch_dense_reg(void* amps, int qubits, int precision, const DenseO
 cudaError_t launch_dense_mma(void* amps, int qubits, const DenseOp& op, const double2* matrix, int sm_count,
                              cudaStream_t st);
 // 6-qubit fused gates on complex64 states of at least 11 qubits run on the tensor cores
-// (qm_dense_tc.cu, 3xTF32) when QM_DENSE_TC=1; otherwise they stay on the FP32 pipes.
+// (qm_dense_tc.cu, 3xTF32) unless QM_DENSE_TC=0 keeps them on the FP32 pipes.
 bool dense_tc_enabled();
 extern std::atomic<int64_t> g_dense_launches, g_dense_tc_launches;  // launch counts (qm_dense_info)
 bool dense_tc_supported(int qubits, int precision, const DenseOp& op);
