@@ -878,8 +878,13 @@ cudaError_t launch_fused(void* amps, int qubits, int precision, const FusedPass&
                          const FusedOp* d_ops, const FusedBatch* batch, cudaStream_t st) {
     if (p.k > qubits || p.op_count > kMaxPassOps || p.op_count < 0 || !d_ops) return cudaErrorInvalidValue;
     if (batch && (batch->states < 1 || batch->states > 65535)) return cudaErrorInvalidValue;
-    bool runs = false;
-    for (int o = p.op_begin + 1; o < p.op_begin + p.op_count; ++o) runs |= (ops[o - 1].flags & ops[o].flags & kOpTurn) != 0;
+    bool runs = false, before = false;
+    for (int o = p.op_begin; o < p.op_begin + p.op_count; ++o) {
+        const bool turn = (ops[o].flags & kOpTurn) != 0;
+        runs |= turn && before;
+        before = turn;
+        if (ops[o].code == OP_DIAG_GROUP) o += (int)ops[o].reserved;  // its members are no run
+    }
     return runs ? launch_fused_t<true>(amps, qubits, precision, p, d_ops, batch, st)
                 : launch_fused_t<false>(amps, qubits, precision, p, d_ops, batch, st);
 }
