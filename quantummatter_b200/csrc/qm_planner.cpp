@@ -768,7 +768,8 @@ bool plan_fused_with(const std::vector<qm_gate>& gates, int qubits, int precisio
 // matrices U_p and U_n, they become H U_p and U_n H and the CNOT a CZ.  A CZ is diagonal, so a
 // stage need not hold t in a register for it and gates commute past it on c and t alike: the
 // 30-qubit brick plans in 25 passes of 142 stages instead of 29 of 185 (complex64: 23 of 130
-// instead of 34 of 191).  Exact up to the rounding of the two matrix products.
+// instead of 34 of 191).  Exact up to one rounding of the two matrix products (with the double nearest to
+// sqrt(1/2) in them, twelve layers of U3 and CNOT at 12 qubits were off by 8.5e-15; 1.0e-15 now).
 bool cz_rewrite_enabled() {
     const char* e = std::getenv("QM_CZ_REWRITE");
     return !(e && e[0] == '0');
@@ -801,7 +802,10 @@ std::vector<qm_gate> cnots_as_cz(const std::vector<qm_gate>& gates) {
                 if (touches(out[i], q)) last[q] = (long)i;
         }
     }
-    const double h = std::sqrt(0.5);
+    // the sums and their product with 1 / sqrt 2 in extended precision, rounded once: the double nearest to
+    // it is 6.8e-17 too large, and each CNOT takes it twice
+    const long double h = 0.707106781186547524400844362104849039L;
+    auto mixed = [&](long double x, long double y) { return (double)(h * (x + y)); };
     for (size_t i = 0; i < n; ++i) {
         const qm_gate& x = out[i];
         if (x.kernel != QM_KERNEL_EXCHANGE || __builtin_popcount(x.control_mask) != 1 || x.swap_control >= 0) continue;
@@ -811,15 +815,15 @@ std::vector<qm_gate> cnots_as_cz(const std::vector<qm_gate>& gates) {
         // H U: rows (a, b) and (c, d) mixed; U H: columns (a, c) and (b, d) mixed
         for (int k = 0; k < 2; ++k) {
             const double a = u.a[k], b = u.b[k], c = u.c[k], d = u.d[k];
-            u.a[k] = h * (a + c);
-            u.b[k] = h * (b + d);
-            u.c[k] = h * (a - c);
-            u.d[k] = h * (b - d);
+            u.a[k] = mixed(a, c);
+            u.b[k] = mixed(b, d);
+            u.c[k] = mixed(a, -c);
+            u.d[k] = mixed(b, -d);
             const double va = v.a[k], vb = v.b[k], vc = v.c[k], vd = v.d[k];
-            v.a[k] = h * (va + vb);
-            v.b[k] = h * (va - vb);
-            v.c[k] = h * (vc + vd);
-            v.d[k] = h * (vc - vd);
+            v.a[k] = mixed(va, vb);
+            v.b[k] = mixed(va, -vb);
+            v.c[k] = mixed(vc, vd);
+            v.d[k] = mixed(vc, -vd);
         }
         u.kernel = QM_KERNEL_MATRIX;
         v.kernel = QM_KERNEL_MATRIX;
